@@ -1,0 +1,695 @@
+// Host path of the operators: argument checks, buffers, plan lookup and launches in native code.
+//
+// A call of an operator costs a few microseconds of GPU time at serving sizes, so what the host does per call decides the
+// rate: the same checks and launches in Python (tensor attributes, a device context manager, ctypes with twenty arguments)
+// took 25 - 45 us per operator and 1.75 ms for the 60 launches of a 12-layer encoder on 128 tokens.  This module takes the
+// Python arguments once, works on at::Tensor, and calls the C ABI (include/stof_b200.h) through function pointers of the
+// library that the ctypes layer loaded; the encoder and decoder stacks walk their layers here without returning to Python.
+//
+// Python keeps what is decided once per mask: the attention plan and its schedule (attention.plan_for_call).  A decided plan
+// is remembered here under the identity of its index tensors, so that later calls find it without Python.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cmath>
+#include <cstdarg>
+#include <cstdio>
+#include <string>
+#include <vector>
+
+#include "../../../include/stof_b200.h"
+
+namespace {
+
+// ------------------------------------------------------------------------------------------ errors
+struct StofFail { std::string text; };
+struct PythonFail {};                        // a Python exception is already set
+
+[[noreturn]] void fail(const char* fmt, ...) {
+    char buf[512];
+    va_list ap;
+    va_start(ap, fmt);
+    vsnprintf(buf, sizeof(buf), fmt, ap);
+    va_end(ap);
+    throw StofFail{buf};
+}
+
+PyObject* g_error = nullptr;                 // StofError
+PyObject* g_status_word = nullptr;           // device index -> int32 tensor
+PyObject* g_plan_for_call = nullptr;         // (index tensors, seq, batch, heads, block_m, block_n) -> (plan, schedule, blocks, final)
+
+template <class F>
+PyObject* guarded(F&& f) {
+    try {
+        return f();
+    } catch (const StofFail& e) {
+        PyErr_SetString(g_error != nullptr ? g_error : PyExc_RuntimeError, e.text.c_str());
+    } catch (const PythonFail&) {
+    } catch (const c10::Error& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return nullptr;
+}
+
+// ------------------------------------------------------------------------------------------ the library
+struct Api {
+    decltype(&stof_last_error) last_error;
+    decltype(&stof_block_attn) block_attn;
+    decltype(&stof_block_attn_scheduled) block_attn_scheduled;
+    decltype(&stof_gemm_bias_act) gemm_bias_act;
+    decltype(&stof_gemm_bias_residual_layernorm) gemm_ln;
+    decltype(&stof_bias_residual_layernorm) layernorm;
+} api = {};
+
+void check(int rc, const char* what) {
+    if (rc != 0) fail("%s failed (code %d): %s", what, rc, api.last_error());
+}
+
+// ------------------------------------------------------------------------------------------ arguments
+// A tensor argument (nullptr for None); anything else is a TypeError.
+const at::Tensor* tensor_arg(PyObject* o, const char* what) {
+    if (o == Py_None) return nullptr;
+    if (!THPVariable_Check(o)) {
+        PyErr_Format(PyExc_TypeError, "%s: a tensor expected, got %s", what, Py_TYPE(o)->tp_name);
+        throw PythonFail{};
+    }
+    return &THPVariable_Unpack(o);
+}
+const at::Tensor& tensor_needed(PyObject* o, const char* what) {
+    const at::Tensor* t = tensor_arg(o, what);
+    if (t == nullptr) {
+        PyErr_Format(PyExc_TypeError, "%s: a tensor expected, got None", what);
+        throw PythonFail{};
+    }
+    return *t;
+}
+long long_arg(PyObject* o) {
+    const long v = PyLong_AsLong(o);
+    if (v == -1 && PyErr_Occurred()) throw PythonFail{};
+    return v;
+}
+double double_arg(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw PythonFail{};
+    return v;
+}
+void need_args(Py_ssize_t got, Py_ssize_t want, const char* what) {
+    if (got != want) {
+        PyErr_Format(PyExc_TypeError, "%s: %zd arguments expected, got %zd", what, want, got);
+        throw PythonFail{};
+    }
+}
+PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
+PyObject* same(PyObject* o) {
+    Py_INCREF(o);
+    return o;
+}
+
+inline bool is_half(const at::Tensor& t) { return t.scalar_type() == at::kHalf; }
+void need_cuda(const at::Tensor* t) {
+    if (t != nullptr && !t->is_cuda()) fail("stof_b200 operators need CUDA tensors (there is no CPU fallback)");
+}
+
+// ------------------------------------------------------------------------------------------ device, stream, status word
+constexpr int MAX_DEVICES = 64;
+int* g_status_ptr[MAX_DEVICES] = {};         // the words are tensors that the Python layer keeps for good
+
+int* status_ptr(int dev) {
+    if (dev < 0 || dev >= MAX_DEVICES) fail("device ordinal %d out of range", dev);
+    if (g_status_ptr[dev] == nullptr) {
+        PyObject* w = PyObject_CallFunction(g_status_word, "i", dev);
+        if (w == nullptr) throw PythonFail{};
+        g_status_ptr[dev] = static_cast<int*>(tensor_needed(w, "status word").data_ptr());
+        Py_DECREF(w);
+    }
+    return g_status_ptr[dev];
+}
+
+struct Launch {                              // device made current, its current stream, its status word
+    c10::cuda::CUDAGuard guard;
+    void* stream;
+    int* status;
+    explicit Launch(const at::Tensor& t)
+        : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.get_device()).stream()), status(status_ptr(t.get_device())) {}
+};
+
+// ------------------------------------------------------------------------------------------ matrices
+struct Rows {                                // a (..., C) tensor seen as rows of C with a contiguous last dimension
+    at::Tensor keep;                         // the copy, where one had to be made
+    const void* ptr;
+    int64_t rows, cols, ld;
+};
+Rows as_rows(const at::Tensor& t) {
+    Rows r;
+    const int64_t d = t.dim();
+    if (d == 0) fail("a tensor with at least one dimension expected");
+    r.cols = t.size(d - 1);
+    if (t.is_contiguous()) {
+        r.rows = r.cols > 0 ? t.numel() / r.cols : 0;
+        r.ld = d == 1 ? r.cols : (d == 2 ? t.stride(0) : r.cols);
+        if (r.rows <= 1 && r.ld < r.cols) r.ld = r.cols;
+        r.ptr = t.data_ptr();
+        return r;
+    }
+    r.keep = (t.stride(d - 1) != 1 ? t.contiguous() : t).reshape({-1, r.cols});
+    r.rows = r.keep.size(0);
+    r.ld = r.keep.stride(0);
+    r.ptr = r.keep.data_ptr();
+    return r;
+}
+
+// A (N) vector operand of a fused operator: fp16, any shape with N elements.  A copy, where one is needed, goes into `keep`.
+const void* vector_arg(const at::Tensor* v, int64_t n, at::Tensor& keep, const char* text) {
+    if (v == nullptr) return nullptr;
+    if (v->numel() != n || !is_half(*v)) fail("%s", text);
+    if (v->is_contiguous()) return v->data_ptr();
+    keep = v->reshape({-1}).contiguous();
+    return keep.data_ptr();
+}
+
+// The output: made here, or the caller's, which has to be viewable as contiguous rows
+struct Out {
+    at::Tensor made;
+    void* ptr;
+    int64_t ld;
+};
+Out output_rows(const at::Tensor* out, const at::Tensor& like, int64_t rows, int64_t cols, const char* op) {
+    Out o;
+    if (out == nullptr) {
+        c10::SmallVector<int64_t, 5> shape(like.sizes().begin(), like.sizes().end());
+        shape.back() = cols;
+        o.made = at::empty(shape, like.options().dtype(at::kHalf));
+        o.ptr = o.made.data_ptr();
+        o.ld = cols;
+        return o;
+    }
+    if (!is_half(*out) || out->numel() != rows * cols || out->dim() == 0 || out->size(-1) != cols)
+        fail("%s: out must be float16 with %lld rows of %lld", op, static_cast<long long>(rows), static_cast<long long>(cols));
+    const Rows r = as_rows(*out);
+    if (r.ptr != out->data_ptr() || (cols > 1 && out->stride(-1) != 1)) fail("%s: output must be viewable as contiguous rows", op);
+    o.ptr = const_cast<void*>(r.ptr);
+    o.ld = r.ld;
+    return o;
+}
+
+struct Weight {
+    at::Tensor keep;
+    const void* ptr;
+    int64_t k, n, ld;
+};
+Weight weight_arg(const at::Tensor& w) {
+    Weight r;
+    r.k = w.size(0);
+    r.n = w.size(1);
+    if (w.stride(1) == 1) {
+        r.ptr = w.data_ptr();
+        r.ld = w.stride(0);
+    } else {
+        r.keep = w.contiguous();
+        r.ptr = r.keep.data_ptr();
+        r.ld = r.keep.stride(0);
+    }
+    return r;
+}
+
+// a (..., K) @ w (K, N) + bias, with an epilogue; the result goes into `out` or a new tensor, which is returned
+at::Tensor gemm_core(const Launch& l, const at::Tensor& a, const at::Tensor& w, const at::Tensor* bias, int epilogue, const at::Tensor* residual,
+                     const at::Tensor* out) {
+    if (!is_half(a) || !is_half(w)) fail("gemm: float16 operands expected");
+    if (w.dim() != 2) fail("gemm: weight must be (K, N)");
+    const Rows x = as_rows(a);
+    const Weight m = weight_arg(w);
+    if (x.cols != m.k) fail("gemm: inner dimensions differ (%lld vs %lld)", static_cast<long long>(x.cols), static_cast<long long>(m.k));
+    at::Tensor kept_bias;
+    const void* b = vector_arg(bias, m.n, kept_bias, "gemm: bias must be a float16 vector of length N");
+    const Out c = output_rows(out, a, x.rows, m.n, "gemm");
+    Rows r{{}, nullptr, 0, 0, 0};
+    if (residual != nullptr) {
+        if (!is_half(*residual)) fail("gemm: residual must be float16 of the output's shape");
+        r = as_rows(*residual);
+        if (r.rows != x.rows || r.cols != m.n) fail("gemm: residual must be float16 of the output's shape");
+    }
+    check(api.gemm_bias_act(x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, c.ptr, c.ld, static_cast<int>(x.rows), static_cast<int>(m.n),
+                            static_cast<int>(m.k), epilogue, l.status, l.stream),
+          "stof_gemm_bias_act");
+    return c.made;
+}
+
+at::Tensor gemm_ln_core(const Launch& l, const at::Tensor& a, const at::Tensor& w, const at::Tensor* bias, const at::Tensor* residual,
+                        const at::Tensor* gamma, const at::Tensor* beta, double eps, const at::Tensor* out) {
+    if (!is_half(a) || !is_half(w) || w.dim() != 2) fail("gemm+layernorm: float16 operands and a (K, N) weight expected");
+    const Rows x = as_rows(a);
+    const Weight m = weight_arg(w);
+    if (x.cols != m.k) fail("gemm+layernorm: inner dimensions differ (%lld vs %lld)", static_cast<long long>(x.cols), static_cast<long long>(m.k));
+    static const char* text = "gemm+layernorm: bias/gamma/beta must be float16 vectors of length N";
+    at::Tensor kept[3];
+    const void* b = vector_arg(bias, m.n, kept[0], text);
+    const void* g = vector_arg(gamma, m.n, kept[1], text);
+    const void* t = vector_arg(beta, m.n, kept[2], text);
+    const Out c = output_rows(out, a, x.rows, m.n, "gemm+layernorm");
+    Rows r{{}, nullptr, 0, 0, 0};
+    if (residual != nullptr) {
+        if (!is_half(*residual)) fail("gemm+layernorm: residual must be float16 of the output's shape");
+        r = as_rows(*residual);
+        if (r.rows != x.rows || r.cols != m.n) fail("gemm+layernorm: residual must be float16 of the output's shape");
+    }
+    check(api.gemm_ln(x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), c.ptr, c.ld, static_cast<int>(x.rows),
+                      static_cast<int>(m.n), static_cast<int>(m.k), l.status, l.stream),
+          "stof_gemm_bias_residual_layernorm");
+    return c.made;
+}
+
+at::Tensor layernorm_core(const Launch& l, const at::Tensor& a, const at::Tensor* bias, const at::Tensor* residual, const at::Tensor* gamma,
+                          const at::Tensor* beta, double eps, const at::Tensor* out) {
+    if (!is_half(a)) fail("layernorm: float16 input expected");
+    const Rows x = as_rows(a);
+    Rows r{{}, nullptr, 0, 0, 0};
+    if (residual != nullptr) {
+        if (!is_half(*residual)) fail("layernorm: residual must be float16 of the input's shape");
+        r = as_rows(*residual);
+        if (r.rows != x.rows || r.cols != x.cols) fail("layernorm: residual must be float16 of the input's shape");
+    }
+    static const char* text = "layernorm: bias/gamma/beta must be float16 vectors of length hidden";
+    at::Tensor kept[3];
+    const void* b = vector_arg(bias, x.cols, kept[0], text);
+    const void* g = vector_arg(gamma, x.cols, kept[1], text);
+    const void* t = vector_arg(beta, x.cols, kept[2], text);
+    const Out y = output_rows(out, a, x.rows, x.cols, "layernorm");
+    check(api.layernorm(x.ptr, x.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), y.ptr, y.ld, static_cast<int>(x.rows),
+                        static_cast<int>(x.cols), l.status, l.stream),
+          "stof_bias_residual_layernorm");
+    return y.made;
+}
+
+// ------------------------------------------------------------------------------------------ attention plans
+// A decided plan under the identity of its index: storage, version counter and length of the four index tensors (which the
+// entry keeps alive, so that no other tensor can take their addresses), shape and block sizes.  Rewrites that torch does not
+// see are announced through forget().  A few dozen entries, the one used last in front.
+struct PlanKey {
+    const void* ptr[4];
+    int64_t version[4], numel[4];
+    int64_t seq, batch, heads, bm, bn, dev;
+    bool operator==(const PlanKey& o) const {
+        for (int i = 0; i < 4; ++i)
+            if (ptr[i] != o.ptr[i] || version[i] != o.version[i] || numel[i] != o.numel[i]) return false;
+        return seq == o.seq && batch == o.batch && heads == o.heads && bm == o.bm && bn == o.bn && dev == o.dev;
+    }
+};
+struct PlanEntry {
+    PlanKey key;
+    at::Tensor index[4], plan, schedule;     // schedule: undefined when the default deal is used
+    int blocks;
+};
+constexpr size_t MAX_PLANS = 32;
+std::vector<PlanEntry>& plans() {
+    static std::vector<PlanEntry>* v = new std::vector<PlanEntry>();     // never destroyed: tensors must not outlive the runtime
+    return *v;
+}
+
+struct Index {
+    const at::Tensor* t[4];                  // full_row_ptr, full_col_idx, part_row_ptr, part_col_idx
+    PyObject* o[4];
+    const at::Tensor* tiles;                 // part_block_mask
+};
+
+PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads, int64_t bm, int64_t bn, int64_t dev) {
+    PlanKey key;
+    bool keyed = true;
+    for (int i = 0; i < 4; ++i) {
+        key.ptr[i] = ix.t[i]->data_ptr();
+        key.numel[i] = ix.t[i]->numel();
+        keyed = keyed && !ix.t[i]->is_inference();
+        key.version[i] = keyed ? static_cast<int64_t>(ix.t[i]->_version()) : 0;
+    }
+    key.seq = seq; key.batch = batch; key.heads = heads; key.bm = bm; key.bn = bn; key.dev = dev;
+    auto& all = plans();
+    if (keyed)
+        for (size_t i = 0; i < all.size(); ++i)
+            if (all[i].key == key) {
+                if (i > 0) std::swap(all[i], all[0]);
+                return all[0];
+            }
+    for (int i = 0; i < 4; ++i)
+        if (ix.t[i]->scalar_type() != at::kInt || !ix.t[i]->is_contiguous()) fail("block attention: index tensors must be contiguous int32");
+    if (key.numel[0] != seq / bm + 1 || key.numel[2] != seq / bm + 1)
+        fail("block attention: row pointer arrays must have S / BLOCK_M + 1 entries");
+    PyObject* r = PyObject_CallFunction(g_plan_for_call, "OOOOLLLLL", ix.o[0], ix.o[1], ix.o[2], ix.o[3], static_cast<long long>(seq),
+                                        static_cast<long long>(batch), static_cast<long long>(heads), static_cast<long long>(bm),
+                                        static_cast<long long>(bn));
+    if (r == nullptr) throw PythonFail{};
+    PyObject *plan, *schedule;
+    int blocks, final_;
+    if (!PyArg_ParseTuple(r, "OOip", &plan, &schedule, &blocks, &final_)) {
+        Py_DECREF(r);
+        throw PythonFail{};
+    }
+    PlanEntry e;
+    e.key = key;
+    for (int i = 0; i < 4; ++i) e.index[i] = *ix.t[i];
+    e.plan = tensor_needed(plan, "plan");
+    if (schedule != Py_None) e.schedule = tensor_needed(schedule, "schedule");
+    e.blocks = blocks;
+    Py_DECREF(r);
+    if (keyed && final_) {
+        if (all.size() >= MAX_PLANS) all.pop_back();
+        all.insert(all.begin(), e);
+    }
+    return e;
+}
+
+struct HeadView {                            // a (B, H, S, 64) view
+    void* ptr;
+    long long stride[3];
+};
+
+void attention_launch(const Launch& l, const PlanEntry& e, const HeadView& q, const HeadView& k, const HeadView& v, const HeadView& out,
+                      const at::Tensor* tiles, int head_dim, float scale) {
+    const int B = static_cast<int>(e.key.batch), H = static_cast<int>(e.key.heads), S = static_cast<int>(e.key.seq);
+    const int bm = static_cast<int>(e.key.bm), bn = static_cast<int>(e.key.bn);
+    const int* prp = static_cast<const int*>(e.index[2].data_ptr());
+    const void* pbm = tiles != nullptr ? tiles->data_ptr() : nullptr;
+    const int rc = e.schedule.defined()
+        ? api.block_attn_scheduled(q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride, prp, pbm,
+                                   e.plan.data_ptr(), bm, bn, 4, scale, static_cast<const int*>(e.schedule.data_ptr()), e.blocks, l.status, l.stream)
+        : api.block_attn(q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride, prp, pbm,
+                         e.plan.data_ptr(), bm, bn, 4, scale, l.status, l.stream);
+    check(rc, "stof_block_attn");
+}
+
+Index index_args(PyObject* const* a) {
+    Index ix;
+    for (int i = 0; i < 4; ++i) {
+        ix.o[i] = a[i];
+        ix.t[i] = &tensor_needed(a[i], "block index");
+    }
+    ix.tiles = tensor_arg(a[4], "part_block_mask");
+    need_cuda(ix.t[0]);
+    need_cuda(ix.t[2]);
+    if (ix.tiles != nullptr && (!is_half(*ix.tiles) || !ix.tiles->is_contiguous()))
+        fail("block attention: part_block_mask must be contiguous float16");
+    return ix;
+}
+
+HeadView head_view(const at::Tensor& t) {
+    return HeadView{t.data_ptr(), {t.stride(0), t.stride(1), t.stride(2)}};
+}
+
+void attention_core(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out, const Index& ix, int64_t bm, int64_t bn,
+                    double scale) {
+    const at::Tensor* all[4] = {&q, &k, &v, &out};
+    for (const at::Tensor* t : all) need_cuda(t);
+    for (const at::Tensor* t : all)
+        if (!is_half(*t)) fail("block attention expects float16 q/k/v/out");
+    if (q.dim() != 4) fail("block attention: q must be (B,H,S,D)");
+    for (const at::Tensor* t : all) {
+        if (t->sizes() != q.sizes()) fail("block attention: q, k, v and out must share one (B,H,S,D) shape");
+        if (t->stride(3) != 1) fail("block attention: the head dimension must be contiguous");
+    }
+    if (bm <= 0 || bn <= 0) fail("block attention: block sizes must be positive");
+    if (scale < 0) scale = 1.0 / std::sqrt(static_cast<double>(q.size(3)));          // src/ops/src/block_attn_mask.cpp:32
+    const Launch l(q);
+    const PlanEntry e = plan_lookup(ix, q.size(2), q.size(0), q.size(1), bm, bn, q.get_device());
+    attention_launch(l, e, head_view(q), head_view(k), head_view(v), head_view(out), ix.tiles, static_cast<int>(q.size(3)),
+                     static_cast<float>(scale));
+}
+
+// ------------------------------------------------------------------------------------------ Python entry points
+// gemm(a, w, bias, epilogue, residual, out) -> out
+PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 6, "gemm");
+        const at::Tensor &x = tensor_needed(a[0], "gemm"), &w = tensor_needed(a[1], "gemm");
+        const at::Tensor *bias = tensor_arg(a[2], "gemm"), *res = tensor_arg(a[4], "gemm"), *out = tensor_arg(a[5], "gemm");
+        for (const at::Tensor* t : {&x, &w, bias, res, out}) need_cuda(t);
+        const Launch l(x);
+        const at::Tensor made = gemm_core(l, x, w, bias, static_cast<int>(long_arg(a[3])), res, out);
+        return out != nullptr ? same(a[5]) : wrap(made);
+    });
+}
+
+// gemm_ln(a, w, bias, residual, gamma, beta, eps, out) -> out
+PyObject* py_gemm_ln(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 8, "gemm_ln");
+        const at::Tensor &x = tensor_needed(a[0], "gemm_ln"), &w = tensor_needed(a[1], "gemm_ln");
+        const at::Tensor *v[4], *out = tensor_arg(a[7], "gemm_ln");
+        for (int i = 0; i < 4; ++i) v[i] = tensor_arg(a[2 + i], "gemm_ln");
+        for (const at::Tensor* t : {&x, &w, v[0], v[1], v[2], v[3], out}) need_cuda(t);
+        const Launch l(x);
+        const at::Tensor made = gemm_ln_core(l, x, w, v[0], v[1], v[2], v[3], double_arg(a[6]), out);
+        return out != nullptr ? same(a[7]) : wrap(made);
+    });
+}
+
+// layernorm(x, bias, residual, gamma, beta, eps, out) -> out
+PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 7, "layernorm");
+        const at::Tensor& x = tensor_needed(a[0], "layernorm");
+        const at::Tensor *v[4], *out = tensor_arg(a[6], "layernorm");
+        for (int i = 0; i < 4; ++i) v[i] = tensor_arg(a[1 + i], "layernorm");
+        for (const at::Tensor* t : {&x, v[0], v[1], v[2], v[3], out}) need_cuda(t);
+        const Launch l(x);
+        const at::Tensor made = layernorm_core(l, x, v[0], v[1], v[2], v[3], double_arg(a[5]), out);
+        return out != nullptr ? same(a[6]) : wrap(made);
+    });
+}
+
+// attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, block_m, block_n, scale) -> out;
+// a negative scale stands for 1 / sqrt(head_dim)
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 12, "attention");
+        attention_core(tensor_needed(a[0], "attention"), tensor_needed(a[1], "attention"), tensor_needed(a[2], "attention"),
+                       tensor_needed(a[3], "attention"), index_args(a + 4), long_arg(a[9]), long_arg(a[10]), double_arg(a[11]));
+        return same(a[3]);
+    });
+}
+
+// attention_inplace(q, k, v, five index tensors, block_m, block_n) -> q, overwritten
+PyObject* py_attention_inplace(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 10, "attention_inplace");
+        const at::Tensor &q = tensor_needed(a[0], "attention"), &k = tensor_needed(a[1], "attention"), &v = tensor_needed(a[2], "attention");
+        if (!q.is_contiguous()) fail("block_attn_mask: q must be contiguous (it is overwritten in place)");
+        const at::Tensor kc = k.contiguous(), vc = v.contiguous();
+        Index ix;
+        at::Tensor kept[5];
+        PyObject* made[5] = {};
+        struct Release {
+            PyObject** p;
+            ~Release() { for (int i = 0; i < 5; ++i) Py_XDECREF(p[i]); }
+        } release{made};
+        PyObject* args[5];
+        for (int i = 0; i < 5; ++i) {
+            const at::Tensor& t = tensor_needed(a[3 + i], "block index");
+            args[i] = a[3 + i];
+            if (!t.is_contiguous()) args[i] = made[i] = wrap(t.contiguous());
+        }
+        attention_core(q, kc, vc, q, index_args(args), long_arg(a[8]), long_arg(a[9]), -1.0);
+        return same(a[0]);
+    });
+}
+
+// merged_attention(q, k, v, result or None, five index tensors, block_m, block_n) -> (B, S, H * D) result
+PyObject* py_merged_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 11, "merged_attention");
+        const at::Tensor &q = tensor_needed(a[0], "attention"), &k = tensor_needed(a[1], "attention"), &v = tensor_needed(a[2], "attention");
+        const at::Tensor* result = tensor_arg(a[3], "attention");
+        for (const at::Tensor* t : {&q, &k, &v, result}) need_cuda(t);
+        if (q.dim() != 4) fail("row-wise attention: q must be (B,H,S,D)");
+        const int64_t B = q.size(0), H = q.size(1), S = q.size(2), D = q.size(3);
+        at::Tensor made;
+        if (result == nullptr) {
+            made = at::empty({B, S, H * D}, q.options());
+        } else if (result->sizes() != at::IntArrayRef({B, S, H * D}) || !result->is_contiguous()) {
+            fail("row-wise attention: result must be a contiguous (batch, S, heads*64) tensor");
+        }
+        const at::Tensor& r = result != nullptr ? *result : made;
+        attention_core(q, k, v, r.as_strided({B, H, S, D}, {S * H * D, D, H * D, 1}), index_args(a + 4), long_arg(a[9]), long_arg(a[10]), -1.0);
+        return result != nullptr ? same(a[3]) : wrap(made);
+    });
+}
+
+// forget(data_ptr): the index tensor at this address was rewritten behind torch's back
+PyObject* py_forget(PyObject*, PyObject* arg) {
+    const void* p = PyLong_AsVoidPtr(arg);
+    if (p == nullptr && PyErr_Occurred()) return nullptr;
+    auto& all = plans();
+    for (size_t i = all.size(); i-- > 0;)
+        for (int j = 0; j < 4; ++j)
+            if (all[i].key.ptr[j] == p) {
+                all.erase(all.begin() + static_cast<long>(i));
+                break;
+            }
+    Py_RETURN_NONE;
+}
+
+// ------------------------------------------------------------------------------------------ encoder and decoder stacks
+// A layer's weights, by attribute name, as tensors (the objects stay alive in the layer)
+struct LayerReader {
+    PyObject* layer;
+    at::Tensor operator()(PyObject* name) const {
+        PyObject* o = PyObject_GetAttr(layer, name);
+        if (o == nullptr) throw PythonFail{};
+        struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } drop{o};
+        const at::Tensor t = tensor_needed(o, "layer weight");
+        need_cuda(&t);
+        return t;
+    }
+};
+#define STOF_NAME(s) ([] { static PyObject* n = PyUnicode_InternFromString(s); return n; }())
+
+struct Stack {
+    at::Tensor qkv, ctx, inter;
+    at::Tensor y[4];
+    PyObject* y_obj[4];
+    int n_y;
+    Index ix;
+    int64_t heads, bm, bn;
+    double eps;
+};
+
+void attention_sublayer(const Launch& l, const Stack& s, const PlanEntry& plan, const at::Tensor& x, const at::Tensor& wqkv, const at::Tensor& bqkv) {
+    gemm_core(l, x, wqkv, &bqkv, STOF_EPI_BIAS, nullptr, &s.qkv);
+    const long long S = s.ctx.size(1), hid = s.ctx.size(2), D = hid / s.heads;
+    char* base = static_cast<char*>(s.qkv.data_ptr());
+    const HeadView q{base, {S * 3 * hid, D, 3 * hid}};
+    const HeadView k{base + 2 * hid, {S * 3 * hid, D, 3 * hid}};
+    const HeadView v{base + 4 * hid, {S * 3 * hid, D, 3 * hid}};
+    const HeadView o{s.ctx.data_ptr(), {S * hid, D, hid}};
+    attention_launch(l, plan, q, k, v, o, s.ix.tiles, static_cast<int>(D), static_cast<float>(1.0 / std::sqrt(static_cast<double>(D))));
+}
+
+void residual_layernorm(const Launch& l, bool fuse, const at::Tensor& a, const at::Tensor& w, const at::Tensor& bias, const at::Tensor& residual,
+                        const at::Tensor& g, const at::Tensor& b, double eps, const at::Tensor& out) {
+    if (fuse) {
+        gemm_ln_core(l, a, w, &bias, &residual, &g, &b, eps, &out);
+    } else {
+        gemm_core(l, a, w, &bias, STOF_EPI_BIAS_RESIDUAL, &residual, &out);
+        layernorm_core(l, out, nullptr, nullptr, &g, &b, eps, &out);
+    }
+}
+
+// stack(layers, hidden, qkv, ctx, inter, (y buffers), five index tensors, block_m, block_n, heads, eps, activation epilogue,
+//       fuse_layernorm, decoder) -> the buffer that holds the last layer's output
+PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 18, "stack");
+        const at::Tensor& hidden = tensor_needed(a[1], "hidden");
+        need_cuda(&hidden);
+        if (hidden.dim() != 3) fail("encoder: hidden must be (B, S, hidden)");
+        Stack s;
+        s.qkv = tensor_needed(a[2], "qkv");
+        s.ctx = tensor_needed(a[3], "ctx");
+        s.inter = tensor_needed(a[4], "inter");
+        s.n_y = static_cast<int>(PyTuple_GET_SIZE(a[5]));
+        for (int i = 0; i < s.n_y && i < 4; ++i) {
+            s.y_obj[i] = PyTuple_GET_ITEM(a[5], i);
+            s.y[i] = tensor_needed(s.y_obj[i], "y");
+        }
+        s.ix = index_args(a + 6);
+        s.bm = long_arg(a[11]);
+        s.bn = long_arg(a[12]);
+        s.heads = long_arg(a[13]);
+        s.eps = double_arg(a[14]);
+        const int act = static_cast<int>(long_arg(a[15]));
+        const bool fuse = PyObject_IsTrue(a[16]) == 1, decoder = PyObject_IsTrue(a[17]) == 1;
+        const Launch l(hidden);
+        at::Tensor x = hidden;
+        PyObject* x_obj = a[1];
+        int yi = 0;
+        const Py_ssize_t layers = PySequence_Size(a[0]);
+        if (layers < 0) throw PythonFail{};
+        for (Py_ssize_t i = 0; i < layers; ++i) {
+            PyObject* layer = PySequence_GetItem(a[0], i);
+            if (layer == nullptr) throw PythonFail{};
+            struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } drop{layer};
+            const LayerReader w{layer};
+            auto sublayer = [&](PyObject* nqkv, PyObject* nbqkv, PyObject* no, PyObject* nbo, PyObject* ng, PyObject* nb) {
+                // looked up per sublayer: an index used for the first time is planned again, better, at its second use
+                const PlanEntry plan = plan_lookup(s.ix, hidden.size(1), hidden.size(0), s.heads, s.bm, s.bn, hidden.get_device());
+                attention_sublayer(l, s, plan, x, w(nqkv), w(nbqkv));
+                const at::Tensor& out = s.y[yi];
+                residual_layernorm(l, fuse, s.ctx, w(no), w(nbo), x, w(ng), w(nb), s.eps, out);
+                x = out;
+                x_obj = s.y_obj[yi];
+                yi = (yi + 1) % s.n_y;
+            };
+            if (decoder) {
+                sublayer(STOF_NAME("Wqkv_a"), STOF_NAME("bqkv_a"), STOF_NAME("Wo_a"), STOF_NAME("bo_a"), STOF_NAME("g_a"), STOF_NAME("b_a"));
+                sublayer(STOF_NAME("Wqkv_c"), STOF_NAME("bqkv_c"), STOF_NAME("Wo_c"), STOF_NAME("bo_c"), STOF_NAME("g_c"), STOF_NAME("b_c"));
+            } else {
+                sublayer(STOF_NAME("Wqkv"), STOF_NAME("bqkv"), STOF_NAME("Wo"), STOF_NAME("bo"), STOF_NAME("g1"), STOF_NAME("b1"));
+            }
+            const at::Tensor bi1 = w(STOF_NAME("bi1"));
+            gemm_core(l, x, w(STOF_NAME("W1")), &bi1, act, nullptr, &s.inter);
+            const at::Tensor& out = s.y[yi];
+            residual_layernorm(l, fuse, s.inter, w(STOF_NAME("W2")), w(STOF_NAME("bi2")), x, w(STOF_NAME("g2")), w(STOF_NAME("b2")), s.eps, out);
+            x = out;
+            x_obj = s.y_obj[yi];
+            yi = (yi + 1) % s.n_y;
+        }
+        return same(x_obj);
+    });
+}
+
+// ------------------------------------------------------------------------------------------ module
+// bind(library path, StofError, status_word, plan_for_call)
+PyObject* py_bind(PyObject*, PyObject* args) {
+    const char* path;
+    PyObject *err, *status, *plan;
+    if (!PyArg_ParseTuple(args, "sOOO", &path, &err, &status, &plan)) return nullptr;
+    void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+    if (h == nullptr) {
+        PyErr_Format(err, "cannot load %s: %s", path, dlerror());
+        return nullptr;
+    }
+    bool ok = true;
+    auto get = [&](auto& f, const char* name) {
+        f = reinterpret_cast<std::remove_reference_t<decltype(f)>>(dlsym(h, name));
+        if (f == nullptr && ok) {
+            PyErr_Format(err, "%s does not export %s", path, name);
+            ok = false;
+        }
+    };
+    Api x = {};
+    get(x.last_error, "stof_last_error");
+    get(x.block_attn, "stof_block_attn");
+    get(x.block_attn_scheduled, "stof_block_attn_scheduled");
+    get(x.gemm_bias_act, "stof_gemm_bias_act");
+    get(x.gemm_ln, "stof_gemm_bias_residual_layernorm");
+    get(x.layernorm, "stof_bias_residual_layernorm");
+    if (!ok) return nullptr;
+    api = x;
+    g_error = same(err);
+    g_status_word = same(status);
+    g_plan_for_call = same(plan);
+    Py_RETURN_NONE;
+}
+
+#define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    {"bind", py_bind, METH_VARARGS, nullptr},
+    FAST("gemm", py_gemm),
+    FAST("gemm_ln", py_gemm_ln),
+    FAST("layernorm", py_layernorm),
+    FAST("attention", py_attention),
+    FAST("attention_inplace", py_attention_inplace),
+    FAST("merged_attention", py_merged_attention),
+    FAST("stack", py_stack),
+    {"forget", py_forget, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_stof_native", "Host path of the stof_b200 operators.", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__stof_native(void) { return PyModule_Create(&module); }

@@ -57,7 +57,34 @@ class Block_Attn_Mask(Function):
         return q
 
 
-rowwise_attn_full_op = RowWise_Attn_Full.apply
-rowwise_attn_sliding_op = RowWise_Attn_Sliding.apply
-rowwise_attn_mask_op = RowWise_Attn_Mask.apply
-block_attn_mask_op = Block_Attn_Mask.apply
+# The operators are forward-only: with nothing to differentiate the autograd.Function machinery (some 10 us a call) has no effect,
+# and the call goes straight to the implementation.
+def _differentiating(q, k, v):
+    return torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
+
+
+def rowwise_attn_full_op(q, k, v, is_causal=False):
+    if _differentiating(q, k, v):
+        return RowWise_Attn_Full.apply(q, k, v, is_causal)
+    return _rowwise.rowwise_attn_full(q.contiguous(), k.contiguous(), v.contiguous(), is_causal)
+
+
+def rowwise_attn_sliding_op(q, k, v, is_causal, bandwidth):
+    if _differentiating(q, k, v):
+        return RowWise_Attn_Sliding.apply(q, k, v, is_causal, bandwidth)
+    return _rowwise.rowwise_attn_sliding(q.contiguous(), k.contiguous(), v.contiguous(), is_causal, bandwidth)
+
+
+def rowwise_attn_mask_op(q, k, v, is_causal, row_mask):
+    if _differentiating(q, k, v):
+        return RowWise_Attn_Mask.apply(q, k, v, is_causal, row_mask)
+    return _rowwise.rowwise_attn_mask(q.contiguous(), k.contiguous(), v.contiguous(), is_causal, row_mask.contiguous())
+
+
+def block_attn_mask_op(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, load_row_ptr, load_col_idx,
+                       BLOCK_M, BLOCK_N, num_warps):
+    if _differentiating(q, k, v):
+        return Block_Attn_Mask.apply(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, load_row_ptr,
+                                     load_col_idx, BLOCK_M, BLOCK_N, num_warps)
+    return _block_attn_mask_forward(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, load_row_ptr,
+                                    load_col_idx, BLOCK_M, BLOCK_N, num_warps)

@@ -70,6 +70,27 @@ def lib() -> ctypes.CDLL:
     return L
 
 
+_native = None
+
+
+def native():
+    """The native host path (`csrc/host/stof_native.cpp`), bound once to the library that `lib()` loads.  Raises StofError
+    when it has not been built; nothing else can stand in for it."""
+    global _native
+    if _native is None:
+        lib()
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        try:
+            from . import _stof_native as mod
+        except ImportError as e:
+            raise StofError(f"stof_b200/_stof_native.so is missing or cannot be loaded ({e}): build it with "
+                            "`python sc25-stof-ad_b200/build.py` (there is no fallback path)") from e
+        from .attention import plan_for_call
+        mod.bind(_LIB_PATH, StofError, lambda index: status_word(torch.device("cuda", index)), plan_for_call)
+        _native = mod
+    return _native
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         msg = lib().stof_last_error().decode("utf-8", "replace")

@@ -1,7 +1,6 @@
 """Block-masked multi-head attention (host side of `stof_block_attn`)."""
 from __future__ import annotations
 
-import math
 from collections import OrderedDict
 
 import torch
@@ -24,6 +23,8 @@ def index_rewritten(*tensors):
     for t in tensors:
         if t is not None:
             _INDEX_GENERATION[t.data_ptr()] = _INDEX_GENERATION.get(t.data_ptr(), 0) + 1
+            if _lib._native is not None:
+                _lib._native.forget(t.data_ptr())
 
 
 _PAIR_MIN_GAIN = 0.06                # re-pair the halves only when that lowers the estimated cost by at least this share
@@ -232,6 +233,17 @@ def attention_schedule(plan, seq_len: int, batch: int, heads: int, eager: bool =
     return table, blocks
 
 
+def plan_for_call(full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, seq_len: int, batch: int, heads: int, block_m: int, block_n: int):
+    """What the native host path asks for when it does not know an index yet: (plan, schedule or None, thread blocks of the
+    schedule, decided).  Once decided - the plan's pairing settled and the deal of its items too - the native side keeps the
+    answer for this index and shape and does not come back."""
+    plan = attention_plan(full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, seq_len, block_m, block_n)
+    hot = plan.data_ptr() in _HOT_PLANS
+    schedule, blocks = attention_schedule(plan, seq_len, batch, heads, eager=hot)
+    one_item_each = ((seq_len + 127) // 128) * batch * heads <= 2 * torch.cuda.get_device_properties(plan.device).multi_processor_count
+    return plan, schedule, int(blocks), hot and (schedule is not None or one_item_each)
+
+
 def block_attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,
                     load_row_ptr, load_col_idx, block_m: int, block_n: int, num_warps: int = 4, softmax_scale=None):
     """Runs the attention kernel on (B,H,S,64)-shaped *views*: q, k, v and out may be arbitrary
@@ -240,54 +252,16 @@ def block_attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part
     way), so no transposing copy is needed around the kernel.  `out` may be `q` itself.
     `load_row_ptr` / `load_col_idx` are accepted for signature compatibility (they are the merge of
     the full and partial lists, which is what the kernel's plan is built from)."""
-    _lib.require_cuda(q, k, v, out, full_row_ptr, part_row_ptr)
-    if q.dtype != torch.float16 or k.dtype != torch.float16 or v.dtype != torch.float16 or out.dtype != torch.float16:
-        raise _lib.StofError("block attention expects float16 q/k/v/out")
-    B, H, S, D = q.shape
-    if k.shape != q.shape or v.shape != q.shape or out.shape != q.shape:
-        raise _lib.StofError("block attention: q, k, v and out must share one (B,H,S,D) shape")
-    for t in (q, k, v, out):
-        if t.stride(3) != 1:
-            raise _lib.StofError("block attention: the head dimension must be contiguous")
-    for t in (full_row_ptr, full_col_idx, part_row_ptr, part_col_idx):
-        if t.dtype != torch.int32 or not t.is_contiguous():
-            raise _lib.StofError("block attention: index tensors must be contiguous int32")
-    if full_row_ptr.numel() != S // block_m + 1 or part_row_ptr.numel() != S // block_m + 1:
-        raise _lib.StofError("block attention: row pointer arrays must have S / BLOCK_M + 1 entries")
-    if part_block_mask is not None and (part_block_mask.dtype != torch.float16 or not part_block_mask.is_contiguous()):
-        raise _lib.StofError("block attention: part_block_mask must be contiguous float16")
-    scale = 1.0 / math.sqrt(D) if softmax_scale is None else float(softmax_scale)   # src/ops/src/block_attn_mask.cpp:32
-    dev = q.device
-    L = _lib.lib()
-    plan = attention_plan(full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, S, int(block_m), int(block_n))
-    schedule, sched_blocks = attention_schedule(plan, S, B, H, eager=plan.data_ptr() in _HOT_PLANS)
-    with torch.cuda.device(dev):
-        st = _lib.status_word(dev)
-        if schedule is None:
-            rc = L.stof_block_attn(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), B, H, S, D,
-                                   _lib.strides3(q.stride()[:3]), _lib.strides3(k.stride()[:3]),
-                                   _lib.strides3(v.stride()[:3]), _lib.strides3(out.stride()[:3]),
-                                   _lib.ptr(part_row_ptr), _lib.ptr(part_block_mask), _lib.ptr(plan),
-                                   int(block_m), int(block_n), int(num_warps), scale, _lib.ptr(st), _lib.current_stream_ptr(dev))
-        else:
-            rc = L.stof_block_attn_scheduled(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), B, H, S, D,
-                                             _lib.strides3(q.stride()[:3]), _lib.strides3(k.stride()[:3]),
-                                             _lib.strides3(v.stride()[:3]), _lib.strides3(out.stride()[:3]),
-                                             _lib.ptr(part_row_ptr), _lib.ptr(part_block_mask), _lib.ptr(plan),
-                                             int(block_m), int(block_n), int(num_warps), scale, _lib.ptr(schedule), int(sched_blocks),
-                                             _lib.ptr(st), _lib.current_stream_ptr(dev))
-    _lib.check(rc, "stof_block_attn")
-    return out
+    return (_lib._native or _lib.native()).attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,
+                                                     block_m, block_n, -1.0 if softmax_scale is None else softmax_scale)
 
 
 def block_attn_mask(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,
                     load_row_ptr, load_col_idx, BLOCK_M, BLOCK_N, num_warps):
     """Semantics of the reference extension's `block_attn_mask.forward`
     (src/ops/src/block_attn_mask.cpp:17-49): overwrites `q` with the attention output."""
-    if not q.is_contiguous():
-        raise _lib.StofError("block_attn_mask: q must be contiguous (it is overwritten in place)")
-    return block_attention(q, k.contiguous(), v.contiguous(), q, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx,
-                           part_block_mask.contiguous(), load_row_ptr, load_col_idx, BLOCK_M, BLOCK_N, num_warps)
+    return (_lib._native or _lib.native()).attention_inplace(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,
+                                                             BLOCK_M, BLOCK_N)
 
 
 def tapered_chunks(batch: int, chunk: int, taper: int):

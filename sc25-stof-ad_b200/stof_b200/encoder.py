@@ -9,8 +9,7 @@ from typing import List
 import torch
 
 from . import _lib
-from .attention import block_attention
-from .fused import bias_residual_layernorm, gemm_bias, gemm_bias_act, gemm_bias_residual, gemm_bias_residual_layernorm
+from .fused import EPILOGUES
 from .masks import get_sparse_storage
 
 
@@ -58,6 +57,7 @@ class BertEncoder:
         self.block_m, self.block_n = block_m, block_n
         self._index = None
         self._bufs = {}
+        self._io = {}
 
     def set_mask(self, mask: torch.Tensor):
         """mask: (1 or B, S, S) 0/1; only mask[0] defines the block index, as in the reference."""
@@ -74,47 +74,30 @@ class BertEncoder:
             self._bufs[key] = torch.empty(shape, dtype=torch.float16, device=device)
         return self._bufs[key]
 
-    def forward(self, hidden: torch.Tensor) -> torch.Tensor:
-        if self._index is None:
-            raise _lib.StofError("BertEncoder: call set_mask() or set_index() first")
+    # hidden-state buffers in rotation: while a GEMM writes one, the previous one is still its residual input and the one
+    # before that may be the caller's view of the last result
+    _STATES = 3
+
+    def _activations(self, hidden):
+        """(qkv, ctx, ffn intermediate, hidden states) of this input's shape, made once."""
         B, S, hid = hidden.shape
-        H = self.head_num
-        D = hid // H
-        dev = hidden.device
-        frp, fci, prp, pci, pbm, lrp, lci = self._index
-        x = hidden
-        qkv = self._buf("qkv", (B, S, 3 * hid), dev)
-        ctx = self._buf("ctx", (B, S, hid), dev)
-        ffn = self.layers[0].W1.shape[1]
-        inter = self._buf("inter", (B, S, ffn), dev)
-        # three hidden-state buffers in rotation: while a GEMM writes one, the previous one is still its residual input and the
-        # one before that may be the caller's view of the last result
-        y_bufs = [self._buf("y0", (B, S, hid), dev), self._buf("y1", (B, S, hid), dev), self._buf("y2", (B, S, hid), dev)]
-        assert len(y_bufs) >= 3
-        yi = 0
-        for w in self.layers:
-            gemm_bias(x, w.Wqkv, w.bqkv, out=qkv)
-            q5 = qkv.view(B, S, 3, H, D)
-            q = q5[:, :, 0].permute(0, 2, 1, 3)
-            k = q5[:, :, 1].permute(0, 2, 1, 3)
-            v = q5[:, :, 2].permute(0, 2, 1, 3)
-            o = ctx.view(B, S, H, D).permute(0, 2, 1, 3)
-            block_attention(q, k, v, o, frp, fci, prp, pci, pbm, lrp, lci, self.block_m, self.block_n)
-            y = y_bufs[yi]; yi = (yi + 1) % 3
-            if self.fuse_layernorm:
-                gemm_bias_residual_layernorm(ctx, w.Wo, w.bo, x, w.g1, w.b1, self.eps, out=y)
-            else:
-                gemm_bias_residual(ctx, w.Wo, w.bo, x, out=y)
-                bias_residual_layernorm(y, None, None, w.g1, w.b1, self.eps, out=y)
-            gemm_bias_act(y, w.W1, w.bi1, self.gelu, out=inter)
-            z = y_bufs[yi]; yi = (yi + 1) % 3
-            if self.fuse_layernorm:
-                gemm_bias_residual_layernorm(inter, w.W2, w.bi2, y, w.g2, w.b2, self.eps, out=z)
-            else:
-                gemm_bias_residual(inter, w.W2, w.bi2, y, out=z)
-                bias_residual_layernorm(z, None, None, w.g2, w.b2, self.eps, out=z)
-            x = z
-        return x
+        key = (B, S, hid, self.layers[0].W1.shape[1], hidden.device)
+        io = self._io.get(key)
+        if io is None:
+            dev = hidden.device
+            states = tuple(self._buf(f"y{i}", (B, S, hid), dev) for i in range(self._STATES))
+            io = self._io[key] = (self._buf("qkv", (B, S, 3 * hid), dev), self._buf("ctx", (B, S, hid), dev),
+                                  self._buf("inter", (B, S, key[3]), dev), states)
+        return io
+
+    def _run(self, hidden, decoder):
+        if self._index is None:
+            raise _lib.StofError(f"{type(self).__name__}: call set_mask() or set_index() first")
+        return (_lib._native or _lib.native()).stack(self.layers, hidden, *self._activations(hidden), *self._index[:5], self.block_m, self.block_n,
+                                                     self.head_num, self.eps, EPILOGUES[self.gelu], self.fuse_layernorm, decoder)
+
+    def forward(self, hidden: torch.Tensor) -> torch.Tensor:
+        return self._run(hidden, False)
 
     __call__ = forward
 
@@ -192,36 +175,9 @@ class T5Decoder(BertEncoder):
     def __init__(self, layers: List[T5DecoderWeights], head_num: int, eps: float = 1e-5, block_m: int = 64, block_n: int = 64):
         super().__init__(layers, head_num, eps, "relu", block_m, block_n)
 
+    _STATES = 4
+
     def forward(self, hidden: torch.Tensor) -> torch.Tensor:
-        if self._index is None:
-            raise _lib.StofError("T5Decoder: call set_mask() or set_index() first")
-        B, S, hid = hidden.shape
-        H = self.head_num
-        D = hid // H
-        dev = hidden.device
-        frp, fci, prp, pci, pbm, lrp, lci = self._index
-        qkv = self._buf("qkv", (B, S, 3 * hid), dev)
-        ctx = self._buf("ctx", (B, S, hid), dev)
-        inter = self._buf("inter", (B, S, self.layers[0].W1.shape[1]), dev)
-        ys = [self._buf(f"y{i}", (B, S, hid), dev) for i in range(4)]
-        yi = 0
-
-        def attention_sublayer(x, Wqkv, bqkv, Wo, bo, g, b, out):
-            gemm_bias(x, Wqkv, bqkv, out=qkv)
-            q5 = qkv.view(B, S, 3, H, D)
-            q, k, v = (q5[:, :, i].permute(0, 2, 1, 3) for i in range(3))
-            block_attention(q, k, v, ctx.view(B, S, H, D).permute(0, 2, 1, 3), frp, fci, prp, pci, pbm, lrp, lci, self.block_m, self.block_n)
-            gemm_bias_residual_layernorm(ctx, Wo, bo, x, g, b, self.eps, out=out)
-            return out
-
-        x = hidden
-        for w in self.layers:
-            y = attention_sublayer(x, w.Wqkv_a, w.bqkv_a, w.Wo_a, w.bo_a, w.g_a, w.b_a, ys[yi]); yi = (yi + 1) % 4
-            y2 = attention_sublayer(y, w.Wqkv_c, w.bqkv_c, w.Wo_c, w.bo_c, w.g_c, w.b_c, ys[yi]); yi = (yi + 1) % 4
-            gemm_bias_act(y2, w.W1, w.bi1, "relu", out=inter)
-            z = ys[yi]; yi = (yi + 1) % 4
-            gemm_bias_residual_layernorm(inter, w.W2, w.bi2, y2, w.g2, w.b2, self.eps, out=z)
-            x = z
-        return x
+        return self._run(hidden, True)
 
     __call__ = forward

@@ -1,5 +1,5 @@
 """Fused GEMM / LayerNorm operators (host side of `stof_gemm_bias_act` and
-`stof_bias_residual_layernorm`)."""
+`stof_bias_residual_layernorm`; argument checks and launches are in `csrc/host/stof_native.cpp`)."""
 from __future__ import annotations
 
 import torch
@@ -7,59 +7,13 @@ import torch
 from . import _lib
 
 
-def _as_rows(t: torch.Tensor):
-    """(…, C) tensor -> (rows, C) view with a contiguous last dim, without copying when possible."""
-    if t.stride(-1) != 1:
-        t = t.contiguous()
-    t2 = t.reshape(-1, t.shape[-1])          # a view whenever the leading dims are collapsible
-    return t2
-
-
-def _gemm(a, w, bias, epilogue, residual=None, out=None):
-    _lib.require_cuda(a, w, bias, residual, out)
-    if a.dtype != torch.float16 or w.dtype != torch.float16:
-        raise _lib.StofError("gemm: float16 operands expected")
-    if w.dim() != 2:
-        raise _lib.StofError("gemm: weight must be (K, N)")
-    a2 = _as_rows(a)
-    if w.stride(1) != 1:
-        w = w.contiguous()
-    M, K = a2.shape
-    K2, N = w.shape
-    if K != K2:
-        raise _lib.StofError(f"gemm: inner dimensions differ ({K} vs {K2})")
-    if bias is not None:
-        bias = bias.reshape(-1)
-        if bias.numel() != N or bias.dtype != torch.float16:
-            raise _lib.StofError("gemm: bias must be a float16 vector of length N")
-        bias = bias.contiguous()
-    out_shape = tuple(a.shape[:-1]) + (N,)
-    if out is None:
-        out = torch.empty(out_shape, dtype=torch.float16, device=a.device)
-    elif out.dtype != torch.float16 or out.numel() != M * N or out.shape[-1] != N:
-        raise _lib.StofError(f"gemm: out must be float16 of shape {out_shape}")       # the kernel stores M rows of N whatever out holds
-    c2 = out.reshape(-1, N)
-    if c2.data_ptr() != out.data_ptr() or c2.stride(1) != 1:
-        raise _lib.StofError("gemm: output must be viewable as contiguous rows")
-    r2, ldr = None, 0
-    if residual is not None:
-        r2 = _as_rows(residual)
-        if r2.shape != (M, N) or r2.dtype != torch.float16:
-            raise _lib.StofError("gemm: residual must be float16 of the output's shape")
-        ldr = r2.stride(0)
-    dev = a.device
-    L = _lib.lib()
-    with torch.cuda.device(dev):
-        st = _lib.status_word(dev)
-        rc = L.stof_gemm_bias_act(_lib.ptr(a2), a2.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(bias), _lib.ptr(r2), ldr,
-                                  _lib.ptr(c2), c2.stride(0), M, N, K, epilogue, _lib.ptr(st), _lib.current_stream_ptr(dev))
-    _lib.check(rc, "stof_gemm_bias_act")
-    return out
+EPILOGUES = {"gelu_erf": _lib.EPI_BIAS_GELU_ERF, "erf": _lib.EPI_BIAS_GELU_ERF, "gelu_tanh": _lib.EPI_BIAS_GELU_TANH,
+             "tanh": _lib.EPI_BIAS_GELU_TANH, "relu": _lib.EPI_BIAS_RELU, "none": _lib.EPI_BIAS}
 
 
 def gemm_bias(a, w, bias=None, out=None):
     """a (..., K) @ w (K, N) + bias (N) -> (..., N) fp16 (fp32 accumulation)."""
-    return _gemm(a, w, bias, _lib.EPI_BIAS, out=out)
+    return (_lib._native or _lib.native()).gemm(a, w, bias, _lib.EPI_BIAS, None, out)
 
 
 def gemm_bias_gelu(a, w, bias=None, mode: str = "erf", out=None):
@@ -67,63 +21,32 @@ def gemm_bias_gelu(a, w, bias=None, mode: str = "erf", out=None):
     "tanh" (src/triton_template/gemm_gemm.py:146-150)."""
     if mode not in ("erf", "tanh"):
         raise _lib.StofError(f"gemm_bias_gelu: unknown mode {mode!r}")
-    return _gemm(a, w, bias, _lib.EPI_BIAS_GELU_ERF if mode == "erf" else _lib.EPI_BIAS_GELU_TANH, out=out)
+    return (_lib._native or _lib.native()).gemm(a, w, bias, _lib.EPI_BIAS_GELU_ERF if mode == "erf" else _lib.EPI_BIAS_GELU_TANH, None, out)
 
 
 def gemm_bias_relu(a, w, bias=None, out=None):
     """GEMM + bias + ReLU in one kernel (the FFN activation of the T5 loops, src/benchmk_end2end.py:203,313)."""
-    return _gemm(a, w, bias, _lib.EPI_BIAS_RELU, out=out)
+    return (_lib._native or _lib.native()).gemm(a, w, bias, _lib.EPI_BIAS_RELU, None, out)
 
 
 def gemm_bias_act(a, w, bias=None, activation: str = "gelu_erf", out=None):
     """GEMM + bias + activation by name: "gelu_erf" (BERT), "gelu_tanh" (GPT-2 `new_gelu`), "relu" (T5), "none"."""
-    epi = {"gelu_erf": _lib.EPI_BIAS_GELU_ERF, "erf": _lib.EPI_BIAS_GELU_ERF, "gelu_tanh": _lib.EPI_BIAS_GELU_TANH,
-           "tanh": _lib.EPI_BIAS_GELU_TANH, "relu": _lib.EPI_BIAS_RELU, "none": _lib.EPI_BIAS}.get(activation)
+    epi = EPILOGUES.get(activation)
     if epi is None:
         raise _lib.StofError(f"gemm_bias_act: unknown activation {activation!r}")
-    return _gemm(a, w, bias, epi, out=out)
+    return (_lib._native or _lib.native()).gemm(a, w, bias, epi, None, out)
 
 
 def gemm_bias_residual(a, w, bias, residual, out=None):
     """GEMM + bias + residual add in one kernel."""
-    return _gemm(a, w, bias, _lib.EPI_BIAS_RESIDUAL, residual=residual, out=out)
+    if residual is None:
+        raise _lib.StofError("gemm: the residual epilogue needs a residual")
+    return (_lib._native or _lib.native()).gemm(a, w, bias, _lib.EPI_BIAS_RESIDUAL, residual, out)
 
 
 def bias_residual_layernorm(x, bias=None, residual=None, gamma=None, beta=None, eps: float = 1e-5, out=None):
     """y = LayerNorm(x + bias + residual) * gamma + beta over the last dimension, one pass over HBM."""
-    _lib.require_cuda(x, bias, residual, gamma, beta, out)
-    if x.dtype != torch.float16:
-        raise _lib.StofError("layernorm: float16 input expected")
-    x2 = _as_rows(x)
-    rows, hidden = x2.shape
-    r2, ldr = None, 0
-    if residual is not None:
-        r2 = _as_rows(residual)
-        if r2.shape != x2.shape or r2.dtype != torch.float16:
-            raise _lib.StofError("layernorm: residual must be float16 of the input's shape")
-        ldr = r2.stride(0)
-    vecs = []
-    for v in (bias, gamma, beta):
-        if v is not None:
-            v = v.reshape(-1).contiguous()
-            if v.numel() != hidden or v.dtype != torch.float16:
-                raise _lib.StofError("layernorm: bias/gamma/beta must be float16 vectors of length hidden")
-        vecs.append(v)
-    if out is None:
-        out = torch.empty(x.shape, dtype=torch.float16, device=x.device)
-    elif out.dtype != torch.float16 or out.numel() != rows * hidden or out.shape[-1] != hidden:
-        raise _lib.StofError(f"layernorm: out must be float16 of shape {tuple(x.shape)}")
-    y2 = out.reshape(-1, hidden)
-    if y2.data_ptr() != out.data_ptr() or y2.stride(1) != 1:
-        raise _lib.StofError("layernorm: output must be viewable as contiguous rows")
-    dev = x.device
-    L = _lib.lib()
-    with torch.cuda.device(dev):
-        rc = L.stof_bias_residual_layernorm(_lib.ptr(x2), x2.stride(0), _lib.ptr(vecs[0]), _lib.ptr(r2), ldr, _lib.ptr(vecs[1]),
-                                            _lib.ptr(vecs[2]), float(eps), _lib.ptr(y2), y2.stride(0), rows, hidden,
-                                            _lib.ptr(_lib.status_word(dev)), _lib.current_stream_ptr(dev))
-    _lib.check(rc, "stof_bias_residual_layernorm")
-    return out
+    return (_lib._native or _lib.native()).layernorm(x, bias, residual, gamma, beta, eps, out)
 
 
 def gemm_bias_residual_layernorm(a, w, bias, residual, gamma, beta, eps: float, out=None):
@@ -132,45 +55,7 @@ def gemm_bias_residual_layernorm(a, w, bias, residual, gamma, beta, eps: float, 
     kernel whose epilogue takes the row statistics across a cluster of thread blocks (`stof_gemm_bias_residual_layernorm`); other
     shapes run the GEMM with the bias + residual epilogue and the LayerNorm kernel in place, behind the same entry point.
     bias, residual, gamma, beta may be None."""
-    _lib.require_cuda(a, w, bias, residual, gamma, beta, out)
-    if a.dtype != torch.float16 or w.dtype != torch.float16 or w.dim() != 2:
-        raise _lib.StofError("gemm+layernorm: float16 operands and a (K, N) weight expected")
-    a2 = _as_rows(a)
-    if w.stride(1) != 1:
-        w = w.contiguous()
-    M, K = a2.shape
-    K2, N = w.shape
-    if K != K2:
-        raise _lib.StofError(f"gemm+layernorm: inner dimensions differ ({K} vs {K2})")
-    vecs = []
-    for v in (bias, gamma, beta):
-        if v is not None:
-            v = v.reshape(-1).contiguous()
-            if v.numel() != N or v.dtype != torch.float16:
-                raise _lib.StofError("gemm+layernorm: bias/gamma/beta must be float16 vectors of length N")
-        vecs.append(v)
-    out_shape = tuple(a.shape[:-1]) + (N,)
-    if out is None:
-        out = torch.empty(out_shape, dtype=torch.float16, device=a.device)
-    elif out.dtype != torch.float16 or out.numel() != M * N or out.shape[-1] != N:
-        raise _lib.StofError(f"gemm+layernorm: out must be float16 of shape {out_shape}")
-    c2 = out.reshape(-1, N)
-    if c2.data_ptr() != out.data_ptr() or c2.stride(1) != 1:
-        raise _lib.StofError("gemm+layernorm: output must be viewable as contiguous rows")
-    r2, ldr = None, 0
-    if residual is not None:
-        r2 = _as_rows(residual)
-        if r2.shape != (M, N) or r2.dtype != torch.float16:
-            raise _lib.StofError("gemm+layernorm: residual must be float16 of the output's shape")
-        ldr = r2.stride(0)
-    dev = a.device
-    L = _lib.lib()
-    with torch.cuda.device(dev):
-        rc = L.stof_gemm_bias_residual_layernorm(_lib.ptr(a2), a2.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(vecs[0]), _lib.ptr(r2), ldr,
-                                                 _lib.ptr(vecs[1]), _lib.ptr(vecs[2]), float(eps), _lib.ptr(c2), c2.stride(0), M, N, K,
-                                                 _lib.ptr(_lib.status_word(dev)), _lib.current_stream_ptr(dev))
-    _lib.check(rc, "stof_gemm_bias_residual_layernorm")
-    return out
+    return (_lib._native or _lib.native()).gemm_ln(a, w, bias, residual, gamma, beta, eps, out)
 
 
 def gemm_bias_residual_then_layernorm(a, w, bias, residual, gamma, beta, eps: float, out=None):

@@ -18,7 +18,6 @@ from collections import OrderedDict
 import torch
 
 from . import _lib
-from .attention import block_attention
 from .masks import get_sparse_storage
 
 _INDEX_CACHE = OrderedDict()
@@ -52,16 +51,8 @@ def _cached_index(key, build_mask, element_granular=True, keep_alive=None):
 
 
 def _run(q, k, v, index, result=None):
-    _lib.require_cuda(q, k, v)
-    B, H, S, D = q.shape
-    if result is None:
-        result = torch.empty(B, S, H * D, dtype=q.dtype, device=q.device)
-    elif tuple(result.shape) != (B, S, H * D) or not result.is_contiguous():
-        raise _lib.StofError("row-wise attention: result must be a contiguous (batch, S, heads*64) tensor")
-    blk = index[0]
-    out_view = result.view(B, S, H, D).permute(0, 2, 1, 3)              # (B,H,S,D) view of the merged-head buffer
-    block_attention(q, k, v, out_view, *index[1:], blk, blk)
-    return result
+    """The attention writes the merged-head (batch, S, heads * 64) layout through its output strides."""
+    return (_lib._native or _lib.native()).merged_attention(q, k, v, result, *index[1:6], index[0], index[0])
 
 
 def _key_range_mask(seq_len, device, lower_exclusive, causal):
@@ -79,7 +70,7 @@ def _key_range_mask(seq_len, device, lower_exclusive, causal):
 def rowwise_attn_full(q, k, v, is_causal=False, result=None):
     """softmax(QK^T / sqrt(64)) V over all keys, or keys <= row when causal; merged-head output."""
     S = q.shape[2]
-    key = ("full", S, bool(is_causal), str(q.device))
+    key = ("full", S, bool(is_causal), q.device)
     index = _cached_index(key, lambda: _key_range_mask(S, q.device, None, bool(is_causal)), element_granular=bool(is_causal))
     return _run(q, k, v, index, result)
 
@@ -87,7 +78,7 @@ def rowwise_attn_full(q, k, v, is_causal=False, result=None):
 def rowwise_attn_sliding(q, k, v, is_causal, bandwidth, result=None):
     """Keys with row - bandwidth < col <= (row if causal else S-1) (src/ops/src/rowwise_attn_sliding_cuda.cu:37,44)."""
     S = q.shape[2]
-    key = ("sliding", S, bool(is_causal), int(bandwidth), str(q.device))
+    key = ("sliding", S, bool(is_causal), int(bandwidth), q.device)
     index = _cached_index(key, lambda: _key_range_mask(S, q.device, int(bandwidth), bool(is_causal)))
     return _run(q, k, v, index, result)
 
@@ -106,6 +97,6 @@ def rowwise_attn_mask(q, k, v, is_causal, row_mask, result=None):
         return allowed.to(device=q.device, dtype=torch.float16).unsqueeze(0)
 
     key = ("mask", S, bool(is_causal), row_mask.data_ptr(), row_mask._version, tuple(row_mask.shape), tuple(row_mask.stride()),
-           str(row_mask.dtype), str(row_mask.device), str(q.device))
+           row_mask.dtype, row_mask.device, q.device)
     index = _cached_index(key, build, keep_alive=row_mask)
     return _run(q, k, v, index, result)
