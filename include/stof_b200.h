@@ -176,11 +176,12 @@ int stof_block_attn_scheduled(const void* q, const void* k, const void* v, void*
  * epilogue: STOF_EPI_BIAS, _GELU_ERF, _GELU_TANH, _RESIDUAL (adds residual[M,N], row stride ldr), _RELU
  * (max(x, 0): the FFN activation of the T5 loops, src/benchmk_end2end.py:203,313).
  * bias may be NULL.
- * Two kernels serve the call: shapes with at least two 256 x 256 tiles per pair of multiprocessors run on
- * pairs of thread blocks (tcgen05 cta_group::2, clusters of two), smaller ones - and residual epilogues with
- * K <= 1024 below 16 such tiles per pair - on single blocks with 128 x 256 tiles; the results agree within
- * fp16 rounding.  The
- * environment variable STOF_B200_GEMM_PAIR = 0 / 1, read once per process, forces one of the two
+ * Three kernels serve the call: shapes whose 64 x 64, 128 x 64 or 128 x 128 tiles all run at once (few rows) on the
+ * small-tile kernel, long contractions there cut over clusters of two or four thread blocks; shapes with at least two
+ * 256 x 256 tiles per pair of multiprocessors on pairs of thread blocks (tcgen05 cta_group::2, clusters of two); those
+ * between - and residual epilogues with K <= 1024 below 16 such tiles per pair - on single blocks with 128 x 256 tiles.
+ * The results agree within fp16 rounding.  The
+ * environment variable STOF_B200_GEMM_PAIR = 0 / 1, read once per process, forces one of the latter two
  * (a testing aid).  GELU_ERF evaluates x * Phi(x) with a polynomial (|error| < 1.1e-4).
  * ------------------------------------------------------------------------------------------ */
 #define STOF_EPI_BIAS 0
@@ -199,8 +200,8 @@ int stof_gemm_bias_act(const void* a, long long lda, const void* w, long long ld
  * Replaces: triton_matmul_bias_layernorm, src/triton_template/gemm_add_layernorm.py:77-144 (statistics inside the
  *           GEMM kernel), and matmul + bias + residual + F.layer_norm of src/benchmk_end2end.py:73-76, 83-86.
  * bias, residual, gamma, beta may be NULL (0 / 0 / 1 / 0).  For n a multiple of 256 up to 1024 and k <= 2048
- * this is ONE kernel (the n / 256 thread blocks of a row block form a cluster and exchange row statistics
- * through distributed shared memory); other shapes run stof_gemm_bias_act followed by
+ * this is ONE kernel (the thread blocks of a row block - n / 256 of them, or n / 64 or n / 128 at few rows - form a
+ * cluster and exchange row statistics through distributed shared memory); other shapes run stof_gemm_bias_act followed by
  * stof_bias_residual_layernorm in place (for long contractions that is the faster of the two, measured).
  * ------------------------------------------------------------------------------------------ */
 int stof_gemm_bias_residual_layernorm(const void* a, long long lda, const void* w, long long ldw, const void* bias,

@@ -512,9 +512,6 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int2* plan_halves = reinterpret_cast<const int2*>(p.plan + plan_off_halves(p.n_qtiles, p.max_steps));
 
     if (threadIdx.x == 0) {
-        // a plan made for another sequence length or block shape is reported, not followed
-        const int4 ph = __ldg(reinterpret_cast<const int4*>(p.plan));
-        const int st = p.status != nullptr ? *p.status : 0;
         for (int i = 0; i < A_QBUFS; ++i) {
             mbar_init(&bars[AB_Q_FULL + i], 1);
             mbar_init(&bars[AB_Q_EMPTY + i], 1);
@@ -532,6 +529,10 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         for (int i = 0; i < A_KSLOTS; ++i) mbar_init(&bars[AB_K_EMPTY + i], 1);
         for (int i = 0; i < A_VSLOTS; ++i) mbar_init(&bars[AB_V_EMPTY + i], 1);
         fence_mbar_init();
+        grid_dependency_wait();
+        // a plan made for another sequence length or block shape is reported, not followed
+        const int4 ph = __ldcg(reinterpret_cast<const int4*>(p.plan));
+        const int st = p.status != nullptr ? *p.status : 0;
         const bool plan_ok = ph.x == PLAN_MAGIC && ph.y == p.seq_len && ph.z == p.bm && ph.w == p.bn;
         if (!plan_ok && p.status != nullptr) atomicCAS(p.status, 0, STATUS_BAD_INDEX);
         *abort_flag = (st != 0 || !plan_ok) ? 1 : 0;
@@ -544,6 +545,8 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
+    grid_launch_dependents();
 
     if (*abort_flag == 0) {
         if (warp == 4) {
@@ -1110,8 +1113,8 @@ static int launch_block_attn(const void* q, const void* k, const void* v, void* 
         STOF_REQUIRE((reinterpret_cast<uintptr_t>(schedule) & 3u) == 0, "block_attn: schedule must be 4-byte aligned");
         grid = schedule_blocks;
     }
-    block_attn_kernel<<<static_cast<unsigned>(grid), A_THREADS, A_SMEM_BYTES, stream>>>(mq, mq16, mk, mv, mo, p);
-    STOF_CUDA(cudaGetLastError());
+    LaunchConfig lc(dim3(static_cast<unsigned>(grid)), A_THREADS, A_SMEM_BYTES, stream);
+    STOF_CUDA(cudaLaunchKernelEx(&lc.cfg, block_attn_kernel, mq, mq16, mk, mv, mo, p));
     return STOF_OK;
 }
 

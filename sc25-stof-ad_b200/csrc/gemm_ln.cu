@@ -23,7 +23,7 @@
 // All blocks of a cluster meet at a cluster barrier before they leave: nobody frees shared memory a peer may still write.
 #include <cstdlib>
 #include <atomic>
-#include "stof_host.h"
+#include "gemm_split.h"
 #include "stof_ptx.cuh"
 
 namespace stof {
@@ -114,6 +114,8 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     cluster_sync_all();
     bool run = true;
     for (int i = 0; i < cluster_size; ++i) run = run && peer_abort[i] == 0;
+    grid_dependency_wait();
+    grid_launch_dependents();
 
     if (run) {
         if (warp == L_EPI_WARPS) {
@@ -357,6 +359,13 @@ extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, c
         const uint32_t box[2] = {64, L_BK};
         if (int rc = make_tensor_map_f16(&mw, w, 2, dims, strides, box)) return rc;
     }
+    if (mode == 0) {
+        int done = 0;
+        const int rc = gemm_split_ln_dispatch({a, lda, &mw, static_cast<const __half*>(bias), static_cast<const __half*>(residual), ldr,
+                                               static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(c), ldc, m, n,
+                                               k, status_dev, stream}, &done);
+        if (rc != STOF_OK || done != 0) return rc;
+    }
     {
         const uint64_t dims[2] = {static_cast<uint64_t>(n), static_cast<uint64_t>(m)};
         const uint64_t strides[1] = {static_cast<uint64_t>(ldc) * 2};
@@ -372,24 +381,16 @@ extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, c
     }
     const int cluster = n / L_BN;
     const int tiles_m = (m + L_BM - 1) / L_BM;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>((sm_count() / cluster) * cluster));
-    cfg.blockDim = dim3(L_THREADS);
-    cfg.dynamicSmemBytes = L_SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    LaunchConfig lc(dim3(static_cast<unsigned>((sm_count() / cluster) * cluster)), L_THREADS, L_SMEM, stream, static_cast<unsigned>(cluster));
     // persistent: exactly as many clusters as the GPU keeps resident at once (the SMs of a cluster lie in one processing
     // cluster of the chip, so fewer than SMs / cluster size may fit), cached per device and cluster size
     static std::atomic<int> resident[64][L_MAX_CLUSTER + 1];
     int clusters = (dev >= 0 && dev < 64) ? resident[dev][cluster].load() : 0;
     if (clusters == 0) {
-        STOF_CUDA(cudaOccupancyMaxActiveClusters(&clusters, gemm_ln_kernel, &cfg));
+        cudaLaunchConfig_t query = lc.cfg;
+        query.attrs = &lc.attr[1];                       // the cluster dimension alone
+        query.numAttrs = 1;
+        STOF_CUDA(cudaOccupancyMaxActiveClusters(&clusters, gemm_ln_kernel, &query));
         if (clusters < 1) {
             set_error("gemm+layernorm: no cluster of %d thread blocks fits on this GPU", cluster);
             return STOF_E_LIMIT;
@@ -397,8 +398,8 @@ extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, c
         if (dev >= 0 && dev < 64) resident[dev][cluster].store(clusters);
     }
     if (clusters > tiles_m) clusters = tiles_m;
-    cfg.gridDim = dim3(static_cast<unsigned>(clusters * cluster));
-    STOF_CUDA(cudaLaunchKernelEx(&cfg, gemm_ln_kernel, ma, mw, mc, static_cast<const __half*>(bias), static_cast<const __half*>(residual), ldr,
+    lc.cfg.gridDim = dim3(static_cast<unsigned>(clusters * cluster));
+    STOF_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_ln_kernel, ma, mw, mc, static_cast<const __half*>(bias), static_cast<const __half*>(residual), ldr,
                                  static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, m, n, k, cluster, status_dev));
     return STOF_OK;
 }

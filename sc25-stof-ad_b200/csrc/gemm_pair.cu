@@ -63,7 +63,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 
 template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
+__global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_c,
                  const __half* __restrict__ bias, const __half* __restrict__ residual, long long ldr, int m, int n, int k, int* status) {
     extern __shared__ unsigned char smem_raw[];
@@ -103,6 +103,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     cluster_sync_all();                                       // both blocks' barriers exist before any remote arrive or copy
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
+    grid_launch_dependents();
 
     if (*abort_flag == 0) {
         if (warp == P_EPI_WARPS) {
@@ -286,8 +288,8 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap&
     const int tiles = ((m + 2 * P_BM - 1) / (2 * P_BM)) * ((n + P_BN - 1) / P_BN);
     int pairs = sm_count() / 2;
     if (pairs > tiles) pairs = tiles;
-    gemm_pair_kernel<EPI><<<2 * pairs, P_THREADS, P_SMEM, stream>>>(ma, mw, mc, bias, residual, ldr, m, n, k, status);
-    STOF_CUDA(cudaGetLastError());
+    LaunchConfig lc(dim3(static_cast<unsigned>(2 * pairs)), P_THREADS, P_SMEM, stream, 2);
+    STOF_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_pair_kernel<EPI>, ma, mw, mc, bias, residual, ldr, m, n, k, status));
     return STOF_OK;
 }
 

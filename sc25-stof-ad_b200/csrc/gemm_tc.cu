@@ -12,7 +12,7 @@
 // descriptor, so no transposed copy is ever made.
 #include <cstdlib>
 #include <atomic>
-#include "stof_host.h"
+#include "gemm_split.h"
 #include "stof_ptx.cuh"
 #include "stof_epilogue.cuh"
 
@@ -69,6 +69,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
+    grid_launch_dependents();
 
     if (*abort_flag == 0) {
         if (warp == G_EPI_WARPS) {
@@ -243,8 +245,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mc, 
     const int tiles = ((m + G_BM - 1) / G_BM) * ((n + G_BN - 1) / G_BN);
     int grid = sm_count();
     if (grid > tiles) grid = tiles;
-    gemm_kernel<EPI><<<grid, G_THREADS, G_SMEM, stream>>>(ma, mw, mc, bias, residual, ldr, m, n, k, status);
-    STOF_CUDA(cudaGetLastError());
+    LaunchConfig lc(dim3(static_cast<unsigned>(grid)), G_THREADS, G_SMEM, stream);
+    STOF_CUDA(cudaLaunchKernelEx(&lc.cfg, gemm_kernel<EPI>, ma, mw, mc, bias, residual, ldr, m, n, k, status));
     return STOF_OK;
 }
 
@@ -253,7 +255,6 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mc, 
 // the two-block (cta_group::2) kernel, gemm_pair.cu
 int gemm_pair_dispatch(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mc, const __half* bias, const __half* residual,
                        long long ldr, int m, int n, int k, int epilogue, int* status, cudaStream_t stream);
-
 namespace {
 // 0 = one-block kernel, 1 = two-block kernel, -1 = by shape.  STOF_B200_GEMM_PAIR overrides (read once).
 int pair_mode() {
@@ -296,6 +297,24 @@ extern "C" int stof_gemm_bias_act(const void* a, long long lda, const void* w, l
         const uint32_t box[2] = {64, G_BK};
         if (int rc = make_tensor_map_f16(&mw, w, 2, dims, strides, box)) return rc;
     }
+    const __half *bp = static_cast<const __half*>(bias), *rp = static_cast<const __half*>(residual);
+    if (pair_mode() < 0) {
+        // Few tiles: the smallest tiles that still all run at once, with K cut in two or four where it is long and that still fits
+        // (gemm_split.cu; a second wave of these one-tile blocks costs more than the 128 x 256 tiles of the kernel below).
+        // Measured, weights from HBM, this kernel against the 128 x 256 one: K = 768: 128 rows x 768 columns 64 x 64 3.4 / 9.1 us,
+        // 512 x 2304 128 x 64 5.3 / 8.9, 1000 x 2304 128 x 128 7.3 / 9.0, 512 x 3072 128 x 128 7.8 / 10.5; K = 3072, 768 columns:
+        // 128 rows 64 x 64 in two parts 5.8 / 22.9, 512 rows 64 x 64 8.2 / 21.4, 1000 rows 128 x 64 10.3 / 21.1.
+        const int sms = sm_count();
+        constexpr int SHAPES[3][2] = {{64, 64}, {128, 64}, {128, 128}};
+        for (const auto& t : SHAPES) {
+            const long long tiles = static_cast<long long>((m + t[0] - 1) / t[0]) * ((n + t[1] - 1) / t[1]);
+            if (tiles > sms) continue;
+            int split = 1;
+            if (k >= 2048 && 2 * tiles <= sms) split = 2;
+            if (k >= 4096 && 4 * tiles <= sms) split = 4;
+            return gemm_split_dispatch({a, lda, &mw, bp, rp, ldr, static_cast<__half*>(c), ldc, m, n, k, split, epilogue, status_dev, stream}, t[0], t[1]);
+        }
+    }
     CUtensorMap mc;
     {
         const uint64_t dims[2] = {static_cast<uint64_t>(n), static_cast<uint64_t>(m)};
@@ -303,7 +322,6 @@ extern "C" int stof_gemm_bias_act(const void* a, long long lda, const void* w, l
         const uint32_t box[2] = {64, 32};
         if (int rc = make_tensor_map_f16(&mc, c, 2, dims, strides, box)) return rc;
     }
-    const __half *bp = static_cast<const __half*>(bias), *rp = static_cast<const __half*>(residual);
     {
         // pairs of blocks on 256 x 256 tiles once every pair of SMs gets at least two of them; small problems keep 128 x 256 tiles.
         // The residual epilogue at K <= 1024 outlasts the main loop in both kernels; measured per shape (K = N = 1024 and 768,

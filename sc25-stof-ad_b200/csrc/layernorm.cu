@@ -62,6 +62,8 @@ layernorm_kernel(const __half* x, long long ldx, const __half* __restrict__ bias
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int warps_total = gridDim.x * LN_WARPS;
     int row = blockIdx.x * LN_WARPS + warp;
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (row >= rows) return;
     const int nchunks = hidden >> 3;
     const float inv_n = 1.0f / static_cast<float>(hidden);
@@ -266,7 +268,6 @@ extern "C" int stof_bias_residual_layernorm(const void* x, long long ldx, const 
     STOF_REQUIRE(aligned16(x) && aligned16(y) && aligned16(bias) && aligned16(residual) && aligned16(gamma) && aligned16(beta),
                  "layernorm: pointers must be 16-byte aligned");
     if (rows == 0) return STOF_OK;
-    const dim3 block(LN_WARPS * 32);
     const __half *xp = static_cast<const __half*>(x), *bp = static_cast<const __half*>(bias), *rp = static_cast<const __half*>(residual),
                  *gp = static_cast<const __half*>(gamma), *tp = static_cast<const __half*>(beta);
     __half* yp = static_cast<__half*>(y);
@@ -285,7 +286,8 @@ extern "C" int stof_bias_residual_layernorm(const void* x, long long ldx, const 
         if (per_sm > LN_BLOCKS_PER_SM) per_sm = LN_BLOCKS_PER_SM;                                                                   \
         int blocks = (rows + LN_WARPS - 1) / LN_WARPS;                                                                              \
         if (blocks > sm_count() * per_sm) blocks = sm_count() * per_sm;                                                             \
-        layernorm_kernel<N><<<dim3(blocks), block, ring_smem, stream>>>(xp, ldx, bp, rp, ldr, gp, tp, eps, yp, ldy, rows, hidden, status_dev);   \
+        LaunchConfig lc(dim3(static_cast<unsigned>(blocks)), LN_WARPS * 32, ring_smem, stream);                                     \
+        STOF_CUDA(cudaLaunchKernelEx(&lc.cfg, layernorm_kernel<N>, xp, ldx, bp, rp, ldr, gp, tp, eps, yp, ldy, rows, hidden, status_dev)); \
     } while (0)
     if (hidden <= 256) STOF_LN_LAUNCH(1);
     else if (hidden <= 512) STOF_LN_LAUNCH(2);
@@ -294,6 +296,5 @@ extern "C" int stof_bias_residual_layernorm(const void* x, long long ldx, const 
     else if (hidden <= 2048) STOF_LN_LAUNCH(8);
     else STOF_LN_LAUNCH(0);
 #undef STOF_LN_LAUNCH
-    STOF_CUDA(cudaGetLastError());
     return STOF_OK;
 }

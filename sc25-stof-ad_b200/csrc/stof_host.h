@@ -38,6 +38,27 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 int make_tensor_map_f16(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                         const uint32_t* box);
 
+// Launch configuration of a kernel that starts under the tail of the kernel before it in the stream (programmatic dependent
+// launch; see grid_dependency_wait in stof_ptx.cuh) and, for cluster > 1, in clusters of that many thread blocks along x.
+struct LaunchConfig {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    LaunchConfig(dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, unsigned cluster = 1) {
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = cluster;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cluster > 1 ? 2 : 1;
+    }
+};
+
 int sm_count();   // multiprocessors of the current device (cached per device)
 
 }  // namespace stof

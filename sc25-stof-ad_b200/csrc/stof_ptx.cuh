@@ -34,6 +34,18 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------------------------
+// Dependent launches (stof_host.h: LaunchConfig)
+// ---------------------------------------------------------------------------------
+// Every kernel of the library is launched so that it may become resident while the kernel before it in the stream still runs.
+// It sets itself up (barriers, tensor memory, descriptors), then waits here until that kernel has completed and its writes are
+// visible, and only then reads or writes global memory that a kernel may touch.  EVERY thread block has to come through
+// grid_dependency_wait before it exits: the next kernel's wait covers this one only, and through this one's wait the ones before.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// From here on the next kernel of the stream may be given whatever this one leaves free of the GPU.  Comes after the wait: what
+// lies two launches back or more is then complete before a kernel starts, and only the kernel just before it has to be waited for.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -105,6 +117,52 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const 
     }
 }
 
+// The same operations on shared-memory ADDRESSES, for loops that a whole warp walks with one lane issuing: what a loop keeps in
+// registers is then a 32-bit address that is the same in every lane, with no generic pointer to convert at each step.
+__device__ __forceinline__ void mbar_arrive_expect_tx_addr(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_test_wait_addr(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(MBAR_SUSPEND_HINT_NS)
+        : "memory");
+    return ok != 0;
+}
+// the part of a wait that has to wait; out of line, so that the loops around it stay short
+static __device__ __noinline__ void mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_smem, int* status_gmem, int barrier_id) {
+    const long long t0 = clock64();
+    int spins = 0;
+    while (!mbar_try_wait_addr(bar, parity)) {
+        if ((++spins & 3) == 0) {
+            if (*abort_smem) return;
+            if (clock64() - t0 > WAIT_BUDGET_CYCLES) {
+                *abort_smem = 1;
+                if (status_gmem) atomicCAS(status_gmem, 0, (barrier_id << 8) | STATUS_WAIT_TIMEOUT);
+                return;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void mbar_wait_addr(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int barrier_id) {
+    if (!mbar_test_wait_addr(bar, parity)) mbar_wait_slow(bar, parity, ctx.abort_smem, ctx.status_gmem, barrier_id);
+}
+
 // The same bounded wait without a CTA-wide abort flag, for waits nobody else can satisfy late (a thread's own bulk
 // copy): false when the cycle budget ran out.
 __device__ __forceinline__ bool mbar_wait_budget(uint64_t* bar, uint32_t parity, long long budget_cycles = WAIT_BUDGET_CYCLES) {
@@ -126,7 +184,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 // address of the same shared-memory location in block `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
     uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_addr) {
@@ -134,6 +192,11 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_addr) {
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same without ordering memory, for the way out of a kernel: what the barrier protects is that nobody's shared memory goes away
+// under a peer, and a releasing arrive would first wait for the block's global stores (1000 cycles and more)
+__device__ __forceinline__ void cluster_sync_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 // The bounded wait with cluster-scope acquire: what the arriving threads of OTHER blocks of the cluster wrote into this
 // block's shared memory before their (release.cluster) arrives is visible afterwards.
@@ -175,6 +238,16 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
         : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_addr(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+// brings a tile into L2 only: no register or shared memory takes a value, so it may run ahead of grid_dependency_wait
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
     asm volatile(
@@ -231,6 +304,10 @@ __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sy
 // arrive on an mbarrier once every MMA issued so far by this thread has completed
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void tc_commit_addr(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // D[tmem] (+)= A[smem] * B[smem]

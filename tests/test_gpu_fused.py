@@ -302,3 +302,32 @@ def test_encoder_forward_captured_in_a_cuda_graph():
     assert torch.equal(replay(), want2)
     from stof_b200 import _lib
     _lib.check_status(x.device, "graph replay")
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 2048), (63, 72, 200), (65, 136, 2056), (100, 768, 3000), (130, 712, 4104), (512, 2304, 72), (1000, 2312, 128), (257, 128, 8192)])
+def test_gemm_with_few_tiles_every_epilogue(m, n, k):
+    """Shapes that run on the small-tile kernel: 64 x 64, 128 x 64 and 128 x 128 tiles with ragged edges, K not a multiple of the
+    stage, K in one, two and four parts over a cluster (from 2048 and 4096 on), in-place residual.  fp16 output of fp32 sums."""
+    import stof_b200
+    a, w, b, r = _rand((m, k), 51), _rand((k, n), 52, k ** -0.5), _rand((n,), 53), _rand((m, n), 54)
+    x = a.float() @ w.float() + b.float()
+    ad, wd, bd = a.cuda(), w.cuda(), b.cuda()
+    out = r.cuda()
+    got = {"none": stof_b200.gemm_bias(ad, wd, bd), "gelu_erf": stof_b200.gemm_bias_gelu(ad, wd, bd), "gelu_tanh": stof_b200.gemm_bias_gelu(ad, wd, bd, "tanh"),
+           "relu": stof_b200.gemm_bias_relu(ad, wd, bd), "residual": stof_b200.gemm_bias_residual(ad, wd, bd, out, out=out), "bare": stof_b200.gemm_bias(ad, wd)}
+    want = {"none": x, "gelu_erf": torch.nn.functional.gelu(x), "gelu_tanh": torch.nn.functional.gelu(x, approximate="tanh"), "relu": x.clamp(min=0),
+            "residual": x + r.float(), "bare": x - b.float()}
+    for name in want:
+        assert _err(got[name], want[name]) <= 2e-3 * max(1.0, want[name].abs().max().item()), name
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 256, 8), (65, 768, 136), (129, 1024, 72), (300, 512, 2048), (600, 768, 768), (1100, 256, 64)])
+def test_small_layernorm_epilogue(m, n, k):
+    """GEMM + LayerNorm at row counts whose row blocks all run at once: clusters of 4 to 16 blocks of 64 x 64 and of up to 8 wider
+    ones, ragged last row block."""
+    import stof_b200
+    a, w, b, r = _rand((m, k), 61), _rand((k, n), 62, k ** -0.5), _rand((n,), 63), _rand((m, n), 64)
+    gam, bet = (_rand((n,), 65, 0.3).float() + 1).half(), _rand((n,), 66, 0.3)
+    want = of.gemm_bias_residual_layernorm(a, w, b, r, gam, bet, 1e-12)
+    got = stof_b200.gemm_bias_residual_layernorm(a.cuda(), w.cuda(), b.cuda(), r.cuda(), gam.cuda(), bet.cuda(), 1e-12)
+    assert _err(got, want) <= 2e-3 * max(1.0, want.abs().max().item())
