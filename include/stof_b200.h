@@ -62,6 +62,24 @@ int stof_mask_fill(const void* mask, int mask_dtype, int seq_len, int block_m, i
                    void* part_block_mask, /* fp16 (n_part, block_m, block_n); may be NULL when n_part == 0 */
                    const void* workspace, size_t workspace_bytes, void* stream);
 
+/* Phase 1 for a caller that waits for the counts on the host right away.  No counterpart in the reference (its loop runs on the
+ * host).  The kernel itself writes them, with the status word, into `notice` - host memory the device can write (pinned and
+ * mapped) - and last of all `stamp`, which the host polls for: nothing is copied and the stream is not synchronised.
+ * `nnz_percent` (device) receives 100 * non-zeros / S^2 in fp32.  `header`: 16 bytes of device memory, zero before the first
+ * call, left at zero by every call; calls that may run at the same time need headers of their own.  `workspace` as above (its
+ * header part is not used); phase 2 is stof_mask_fill. */
+typedef struct stof_mask_notice {
+    int n_full, n_part;
+    long long nnz;
+    int status, reserved;
+    unsigned long long stamp;
+} stof_mask_notice;
+
+int stof_mask_classify_notify(const void* mask, int mask_dtype, int batch, int seq_len, int block_m, int block_n,
+                              int* full_row_ptr, int* part_row_ptr, int* load_row_ptr, float* nnz_percent,
+                              void* workspace, size_t workspace_bytes, void* header, const int* status_dev,
+                              stof_mask_notice* notice, unsigned long long stamp, void* stream);
+
 /* Mask compaction for callers that must not allocate.
  * No counterpart in the reference: its get_sparse_storage builds Python lists and allocates freely.
  *

@@ -35,7 +35,7 @@ def _native_command():
     return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"],
             "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
             "-I" + os.path.join(cuda, "include"), NATIVE_SRC, "-o", NATIVE, "-L" + os.path.join(root, "lib"),
-            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+            "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
 
 
 def _stale() -> bool:

@@ -11,14 +11,18 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
+#include <sched.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -41,6 +45,7 @@ struct PythonFail {};                        // a Python exception is already se
 
 PyObject* g_error = nullptr;                 // StofError
 PyObject* g_status_word = nullptr;           // device index -> int32 tensor
+PyObject* g_check_status = nullptr;          // (device index, what): reads the word, clears it and raises
 PyObject* g_plan_for_call = nullptr;         // (index tensors, seq, batch, heads, block_m, block_n) -> (plan, schedule, blocks, final)
 
 template <class F>
@@ -61,6 +66,9 @@ PyObject* guarded(F&& f) {
 // ------------------------------------------------------------------------------------------ the library
 struct Api {
     decltype(&stof_last_error) last_error;
+    decltype(&stof_mask_workspace_bytes) mask_workspace_bytes;
+    decltype(&stof_mask_classify_notify) mask_classify_notify;
+    decltype(&stof_mask_fill) mask_fill;
     decltype(&stof_block_attn) block_attn;
     decltype(&stof_block_attn_scheduled) block_attn_scheduled;
     decltype(&stof_gemm_bias_act) gemm_bias_act;
@@ -140,6 +148,9 @@ struct Launch {                              // device made current, its current
         : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.get_device()).stream()), status(status_ptr(t.get_device())) {}
 };
 
+// A new tensor on t's device, without the dispatcher's round
+at::Tensor make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor& t) { return at::detail::empty_cuda(shape, type, t.device(), std::nullopt); }
+
 // ------------------------------------------------------------------------------------------ matrices
 struct Rows {                                // a (..., C) tensor seen as rows of C with a contiguous last dimension
     at::Tensor keep;                         // the copy, where one had to be made
@@ -185,7 +196,7 @@ Out output_rows(const at::Tensor* out, const at::Tensor& like, int64_t rows, int
     if (out == nullptr) {
         c10::SmallVector<int64_t, 5> shape(like.sizes().begin(), like.sizes().end());
         shape.back() = cols;
-        o.made = at::empty(shape, like.options().dtype(at::kHalf));
+        o.made = make(shape, at::kHalf, like);
         o.ptr = o.made.data_ptr();
         o.ld = cols;
         return o;
@@ -509,7 +520,7 @@ PyObject* py_merged_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t B = q.size(0), H = q.size(1), S = q.size(2), D = q.size(3);
         at::Tensor made;
         if (result == nullptr) {
-            made = at::empty({B, S, H * D}, q.options());
+            made = make({B, S, H * D}, q.scalar_type(), q);
         } else if (result->sizes() != at::IntArrayRef({B, S, H * D}) || !result->is_contiguous()) {
             fail("row-wise attention: result must be a contiguous (batch, S, heads*64) tensor");
         }
@@ -642,12 +653,130 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// ------------------------------------------------------------------------------------------ mask -> block index
+// What a compaction in progress keeps for itself on a device: a header that its kernel leaves at zero and a record in host
+// memory that the kernel writes its counts to.  A fixed number per device, made at its first compaction; a call holds one until
+// it has seen its kernel's stamp, so calls from several threads and on several streams do not meet.
+constexpr int NOTICES = 16;
+struct NoticePool {
+    char* headers = nullptr;                 // device, NOTICES x 16 bytes
+    stof_mask_notice* notices = nullptr;     // pinned host memory
+    unsigned long long stamp = 0;
+    bool busy[NOTICES] = {};
+};
+NoticePool g_notices[MAX_DEVICES];           // guarded by the GIL
+
+void cuda_ok(cudaError_t e, const char* what) {
+    if (e != cudaSuccess) fail("%s failed: %s", what, cudaGetErrorString(e));
+}
+
+struct Notice {
+    NoticePool& pool;
+    int slot = -1;
+    unsigned long long stamp = 0;
+    explicit Notice(int dev) : pool(g_notices[dev]) {
+        if (pool.notices == nullptr) {
+            void *h = nullptr, *n = nullptr;
+            cuda_ok(cudaMalloc(&h, NOTICES * 16), "cudaMalloc");
+            cuda_ok(cudaMemset(h, 0, NOTICES * 16), "cudaMemset");
+            cuda_ok(cudaHostAlloc(&n, NOTICES * sizeof(stof_mask_notice), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+            memset(n, 0, NOTICES * sizeof(stof_mask_notice));
+            cuda_ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+            pool.headers = static_cast<char*>(h);
+            pool.notices = static_cast<stof_mask_notice*>(n);
+        }
+        while (slot < 0) {
+            for (int i = 0; i < NOTICES && slot < 0; ++i)
+                if (!pool.busy[i]) slot = i;
+            if (slot < 0) {                  // sixteen other threads are waiting for theirs
+                PyThreadState* ts = PyEval_SaveThread();
+                sched_yield();
+                PyEval_RestoreThread(ts);
+            }
+        }
+        pool.busy[slot] = true;
+        stamp = ++pool.stamp;
+    }
+    ~Notice() { pool.busy[slot] = false; }
+    void* header() const { return pool.headers + 16 * slot; }
+    stof_mask_notice* record() const { return pool.notices + slot; }
+    // Polls until the kernel has written the stamp.  A stream that fails, or has nothing left to do without having written it,
+    // ends the wait; the GIL is free meanwhile.
+    stof_mask_notice wait(cudaStream_t stream) {
+        volatile unsigned long long* at = &record()->stamp;
+        cudaError_t e = cudaErrorNotReady;
+        PyThreadState* ts = PyEval_SaveThread();
+        for (unsigned spins = 1; *at != stamp; ++spins) {
+            if ((spins & 0x3FFF) != 0) {
+                __builtin_ia32_pause();
+                continue;
+            }
+            e = cudaStreamQuery(stream);
+            if (e != cudaErrorNotReady) break;
+        }
+        PyEval_RestoreThread(ts);
+        if (*at != stamp) {
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (*at != stamp) fail("get_sparse_storage: the compaction did not report: %s", cudaGetErrorString(e));
+        }
+        __sync_synchronize();
+        return *record();
+    }
+};
+
+// sparse_storage(mask (batch, S, S) on the GPU, contiguous, block_m, block_n) -> the eight values of get_sparse_storage
+PyObject* py_sparse_storage(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        need_args(n, 3, "sparse_storage");
+        const at::Tensor& m = tensor_needed(a[0], "mask");
+        need_cuda(&m);
+        const int64_t bm = long_arg(a[1]), bn = long_arg(a[2]), B = m.size(0), S = m.size(2);
+        if (bm <= 0 || bn <= 0 || S % bm != 0 || S % bn != 0)
+            fail("get_sparse_storage: S=%lld must be a multiple of the block sizes (%lld, %lld)", static_cast<long long>(S), static_cast<long long>(bm),
+                 static_cast<long long>(bn));
+        const int dt = is_half(m) ? STOF_DTYPE_F16 : STOF_DTYPE_F32, s = static_cast<int>(S), ibm = static_cast<int>(bm), ibn = static_cast<int>(bn);
+        const Launch l(m);
+        const cudaStream_t stream = static_cast<cudaStream_t>(l.stream);
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        cuda_ok(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing");
+        if (capturing != cudaStreamCaptureStatusNone) fail("get_sparse_storage: the sizes of its outputs depend on the data, so it cannot be captured");
+        const int64_t rows = S / bm + 1;
+        const at::Tensor frp = make({rows}, at::kInt, m), prp = make({rows}, at::kInt, m), lrp = make({rows}, at::kInt, m);
+        const at::Tensor nnz = make({}, at::kFloat, m);
+        const size_t ws_bytes = api.mask_workspace_bytes(s, ibm, ibn);
+        const at::Tensor ws = make({static_cast<int64_t>(ws_bytes)}, at::kByte, m);
+        stof_mask_notice got;
+        {
+            Notice notice(m.get_device());
+            check(api.mask_classify_notify(m.data_ptr(), dt, static_cast<int>(B), s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(),
+                                           nnz.data_ptr<float>(), ws.data_ptr(), ws_bytes, notice.header(), l.status, notice.record(), notice.stamp, l.stream),
+                  "stof_mask_classify");
+            got = notice.wait(stream);
+        }
+        if (got.status != 0) {
+            PyObject* r = PyObject_CallFunction(g_check_status, "is", static_cast<int>(m.get_device()), "a kernel launched before this get_sparse_storage");
+            if (r == nullptr) throw PythonFail{};
+            Py_DECREF(r);
+        }
+        const at::Tensor fci = make({got.n_full}, at::kInt, m), pci = make({got.n_part}, at::kInt, m), lci = make({got.n_full + got.n_part}, at::kInt, m);
+        const at::Tensor tiles = got.n_part > 0 ? make({got.n_part, bm, bn}, at::kHalf, m) : at::ones({1, bm, bn}, m.options().dtype(at::kHalf));
+        if (got.n_full + got.n_part > 0)
+            check(api.mask_fill(m.data_ptr(), dt, s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(), fci.data_ptr<int>(),
+                                pci.data_ptr<int>(), lci.data_ptr<int>(), got.n_part > 0 ? tiles.data_ptr() : nullptr, ws.data_ptr(), ws_bytes, l.stream),
+                  "stof_mask_fill");
+        const at::Tensor* out[8] = {&nnz, &frp, &fci, &prp, &pci, &tiles, &lrp, &lci};
+        PyObject* tuple = PyTuple_New(8);
+        for (int i = 0; i < 8; ++i) PyTuple_SET_ITEM(tuple, i, wrap(*out[i]));
+        return tuple;
+    });
+}
+
 // ------------------------------------------------------------------------------------------ module
-// bind(library path, StofError, status_word, plan_for_call)
+// bind(library path, StofError, status_word, check_status, plan_for_call)
 PyObject* py_bind(PyObject*, PyObject* args) {
     const char* path;
-    PyObject *err, *status, *plan;
-    if (!PyArg_ParseTuple(args, "sOOO", &path, &err, &status, &plan)) return nullptr;
+    PyObject *err, *status, *check_word, *plan;
+    if (!PyArg_ParseTuple(args, "sOOOO", &path, &err, &status, &check_word, &plan)) return nullptr;
     void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
     if (h == nullptr) {
         PyErr_Format(err, "cannot load %s: %s", path, dlerror());
@@ -663,6 +792,9 @@ PyObject* py_bind(PyObject*, PyObject* args) {
     };
     Api x = {};
     get(x.last_error, "stof_last_error");
+    get(x.mask_workspace_bytes, "stof_mask_workspace_bytes");
+    get(x.mask_classify_notify, "stof_mask_classify_notify");
+    get(x.mask_fill, "stof_mask_fill");
     get(x.block_attn, "stof_block_attn");
     get(x.block_attn_scheduled, "stof_block_attn_scheduled");
     get(x.gemm_bias_act, "stof_gemm_bias_act");
@@ -672,6 +804,7 @@ PyObject* py_bind(PyObject*, PyObject* args) {
     api = x;
     g_error = same(err);
     g_status_word = same(status);
+    g_check_status = same(check_word);
     g_plan_for_call = same(plan);
     Py_RETURN_NONE;
 }
@@ -686,6 +819,7 @@ PyMethodDef methods[] = {
     FAST("attention_inplace", py_attention_inplace),
     FAST("merged_attention", py_merged_attention),
     FAST("stack", py_stack),
+    FAST("sparse_storage", py_sparse_storage),
     {"forget", py_forget, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_stof_native", "Host path of the stof_b200 operators.", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -11,7 +11,7 @@ _LIB_PATH = os.environ.get("STOF_B200_LIBRARY") or os.path.join(_HERE, "libstof_
 STOF_DTYPE_F16, STOF_DTYPE_F32 = 0, 1
 EPI_BIAS, EPI_BIAS_GELU_ERF, EPI_BIAS_GELU_TANH, EPI_BIAS_RESIDUAL, EPI_BIAS_RELU = 0, 1, 2, 3, 4
 
-EXPORTS = ("stof_version", "stof_last_error", "stof_mask_workspace_bytes", "stof_mask_classify", "stof_mask_fill", "stof_mask_compact_static",
+EXPORTS = ("stof_version", "stof_last_error", "stof_mask_workspace_bytes", "stof_mask_classify", "stof_mask_classify_notify", "stof_mask_fill", "stof_mask_compact_static",
            "stof_block_attn_plan_bytes", "stof_block_attn_plan", "stof_block_attn_plan_paired", "stof_block_attn", "stof_block_attn_scheduled", "stof_gemm_bias_act", "stof_gemm_bias_residual_layernorm", "stof_bias_residual_layernorm")
 
 
@@ -44,6 +44,8 @@ def lib() -> ctypes.CDLL:
     L.stof_mask_workspace_bytes.argtypes = [i32, i32, i32]
     L.stof_mask_classify.restype = i32
     L.stof_mask_classify.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, sz, vp]
+    L.stof_mask_classify_notify.restype = i32
+    L.stof_mask_classify_notify.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, sz, vp, vp, vp, ctypes.c_ulonglong, vp]
     L.stof_mask_fill.restype = i32
     L.stof_mask_fill.argtypes = [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]
     L.stof_mask_compact_static.restype = i32
@@ -86,7 +88,8 @@ def native():
             raise StofError(f"stof_b200/_stof_native.so is missing or cannot be loaded ({e}): build it with "
                             "`python sc25-stof-ad_b200/build.py` (there is no fallback path)") from e
         from .attention import plan_for_call
-        mod.bind(_LIB_PATH, StofError, lambda index: status_word(torch.device("cuda", index)), plan_for_call)
+        mod.bind(_LIB_PATH, StofError, lambda index: status_word(torch.device("cuda", index)),
+                 lambda index, what: check_status(torch.device("cuda", index), what), plan_for_call)
         _native = mod
     return _native
 

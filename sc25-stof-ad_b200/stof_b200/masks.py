@@ -29,43 +29,9 @@ def get_sparse_storage(Mask: torch.Tensor, block_size_m: int, block_size_n: int)
         raise _lib.StofError("get_sparse_storage expects a (batch, S, S) mask")
     if Mask.dtype not in (torch.float16, torch.float32):
         raise _lib.StofError(f"get_sparse_storage: mask dtype {Mask.dtype} unsupported (float16 or float32)")
-    home = Mask.device
-    m = Mask if Mask.is_cuda else Mask.cuda()
-    m = m.contiguous()
-    dev = m.device
-    B, S = m.shape[0], m.shape[-1]
-    bm, bn = int(block_size_m), int(block_size_n)
-    L = _lib.lib()
-    dt = _lib.STOF_DTYPE_F16 if m.dtype == torch.float16 else _lib.STOF_DTYPE_F32
-    if S % bm or S % bn:
-        raise _lib.StofError(f"get_sparse_storage: S={S} must be a multiple of the block sizes ({bm}, {bn})")
-    nbm = S // bm
-    with torch.cuda.device(dev):
-        stream = _lib.current_stream_ptr(dev)
-        ws_bytes = int(L.stof_mask_workspace_bytes(S, bm, bn))
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        row_ptrs = torch.empty(3, nbm + 1, dtype=torch.int32, device=dev)
-        counts = torch.empty(4, dtype=torch.int64, device=dev)
-        _lib.check(L.stof_mask_classify(_lib.ptr(m), dt, B, S, bm, bn, _lib.ptr(row_ptrs[0]), _lib.ptr(row_ptrs[1]),
-                                        _lib.ptr(row_ptrs[2]), _lib.ptr(counts), _lib.ptr(ws), ws_bytes, stream),
-                   "stof_mask_classify")
-        n_full, n_part, n_load, nnz_elems = counts.tolist()          # the one host read: output sizes depend on the data
-        _lib.check_status(dev, "a kernel launched before this get_sparse_storage")   # the stream is drained here anyway
-        full_col = torch.empty(n_full, dtype=torch.int32, device=dev)
-        part_col = torch.empty(n_part, dtype=torch.int32, device=dev)
-        load_col = torch.empty(n_load, dtype=torch.int32, device=dev)
-        tiles = torch.empty(n_part, bm, bn, dtype=torch.float16, device=dev) if n_part else None
-        _lib.check(L.stof_mask_fill(_lib.ptr(m), dt, S, bm, bn, _lib.ptr(row_ptrs[0]), _lib.ptr(row_ptrs[1]), _lib.ptr(row_ptrs[2]),
-                                    _lib.ptr(full_col), _lib.ptr(part_col), _lib.ptr(load_col), _lib.ptr(tiles),
-                                    _lib.ptr(ws), ws_bytes, stream), "stof_mask_fill")
-        if tiles is None:
-            tiles = torch.ones(1, bm, bn, dtype=torch.float16, device=dev)
-        # same operation order as the reference: int64 count -> / S^2 -> * 100, in float32
-        nnz = torch.tensor(nnz_elems, dtype=torch.int64, device=dev) / (S * S) * 100
-    out = (nnz, row_ptrs[0], full_col, row_ptrs[1], part_col, tiles, row_ptrs[2], load_col)
-    if home != dev:
-        out = tuple(t.to(home) for t in out)
-    return out
+    m = (Mask if Mask.is_cuda else Mask.cuda()).contiguous()
+    out = (_lib._native or _lib.native()).sparse_storage(m, int(block_size_m), int(block_size_n))
+    return out if Mask.is_cuda else tuple(t.to(Mask.device) for t in out)
 
 
 class SparseStorageRefresher:

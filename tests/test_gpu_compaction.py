@@ -1,4 +1,6 @@
 """CUDA mask -> block-index compaction against the oracle and the reference-generated fixtures (bit-exact)."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -113,3 +115,18 @@ def test_refresher_reuses_buffers_and_detects_structure_change():
     ref.refresh()
     with pytest.raises(stof_b200.StofError):
         ref.check()
+
+
+@pytest.mark.parametrize("seq_len,bm,bn,batch", [(64, 64, 64, 1), (200, 8, 8, 3), (528, 16, 176, 2), (4096, 4096, 4096, 1), (2304, 256, 2304, 2), (1040, 208, 16, 1)])
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+def test_compaction_stripe_and_tile_edges(seq_len, bm, bn, batch, dtype):
+    """Tiles wider than a thread block's row of chunks, one single tile, stripes that end short of the mask's edge, rows of class
+    bytes that are not a multiple of sixteen, and non-zeros counted over every batch element."""
+    rng = np.random.default_rng(seq_len + bm)
+    mask = (rng.random((batch, seq_len, seq_len)) < 0.5).astype(dtype)
+    mask[0, :, : bn // 2] = 1
+    mask[0, : seq_len // 2] = 0
+    mask[0, -bm:] = 1
+    got, st = _run(mask, bm, bn), om.get_sparse_storage(mask, bm, bn)
+    share = torch.tensor(np.count_nonzero(mask), device="cuda") / (seq_len * seq_len) * 100        # the same fp32 operations on the GPU
+    _compare(got, dataclasses.replace(st, nnz=share.item()))
