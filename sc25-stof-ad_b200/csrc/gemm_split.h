@@ -40,4 +40,7 @@ struct SplitLnCall {
 // all run at once
 int gemm_split_ln_dispatch(const SplitLnCall& x, int* done);
 
+// gemm_tc.cu: rounds of tiles of the GEMM without LayerNorm, for the choice between one kernel and two
+long long gemm_rounds(int m, int n, int k, int epilogue);
+
 }  // namespace stof

@@ -264,7 +264,25 @@ int pair_mode() {
     }();
     return mode;
 }
+// Pairs of blocks on 256 x 256 tiles once every pair of SMs gets at least two of them; small problems keep 128 x 256 tiles.
+// The residual epilogue at K <= 1024 outlasts the main loop in both kernels; measured per shape (K = N = 1024 and 768,
+// bias + residual): 16384 rows one-block +3 %, 65536 rows equal within 1.5 %, 262144 rows two-block +3 % - so that case
+// moves to the two-block kernel only from 16 tiles per pair of SMs on.
+bool takes_pairs(int m, int n, int k, int epilogue) {
+    const int mode = pair_mode();
+    if (mode >= 0) return mode == 1;
+    const long long tiles256 = ((m + 255LL) / 256) * ((n + 255LL) / 256), pairs = sm_count() / 2;
+    const bool short_residual = epilogue == STOF_EPI_BIAS_RESIDUAL && k <= 1024;
+    return tiles256 >= (short_residual ? 16LL : 2LL) * pairs;
+}
 }  // namespace
+
+// Tiles of 256 columns that the busiest multiprocessor (or pair) walks in the GEMM kernel that a shape gets, small tiles apart
+long long gemm_rounds(int m, int n, int k, int epilogue) {
+    const bool pairs = takes_pairs(m, n, k, epilogue);
+    const long long rows = pairs ? 256 : 128, workers = pairs ? sm_count() / 2 : sm_count();
+    return (((m + rows - 1) / rows) * ((n + 255LL) / 256) + workers - 1) / workers;
+}
 }  // namespace stof
 
 using namespace stof;
@@ -322,18 +340,7 @@ extern "C" int stof_gemm_bias_act(const void* a, long long lda, const void* w, l
         const uint32_t box[2] = {64, 32};
         if (int rc = make_tensor_map_f16(&mc, c, 2, dims, strides, box)) return rc;
     }
-    {
-        // pairs of blocks on 256 x 256 tiles once every pair of SMs gets at least two of them; small problems keep 128 x 256 tiles.
-        // The residual epilogue at K <= 1024 outlasts the main loop in both kernels; measured per shape (K = N = 1024 and 768,
-        // bias + residual): 16384 rows one-block +3 %, 65536 rows equal within 1.5 %, 262144 rows two-block +3 % - so that case
-        // moves to the two-block kernel only from 16 tiles per pair of SMs on.
-        const long long tiles256 = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256);
-        const int mode = pair_mode();
-        const long long pairs = sm_count() / 2;
-        const bool short_residual = epilogue == STOF_EPI_BIAS_RESIDUAL && k <= 1024;
-        if (mode == 1 || (mode < 0 && tiles256 >= (short_residual ? 16LL : 2LL) * pairs))
-            return gemm_pair_dispatch(ma, mw, mc, bp, rp, ldr, m, n, k, epilogue, status_dev, stream);
-    }
+    if (takes_pairs(m, n, k, epilogue)) return gemm_pair_dispatch(ma, mw, mc, bp, rp, ldr, m, n, k, epilogue, status_dev, stream);
     switch (epilogue) {
         case STOF_EPI_BIAS: return launch<STOF_EPI_BIAS>(ma, mw, mc, bp, rp, ldr, m, n, k, status_dev, stream);
         case STOF_EPI_BIAS_GELU_ERF: return launch<STOF_EPI_BIAS_GELU_ERF>(ma, mw, mc, bp, rp, ldr, m, n, k, status_dev, stream);

@@ -331,3 +331,24 @@ def test_small_layernorm_epilogue(m, n, k):
     want = of.gemm_bias_residual_layernorm(a, w, b, r, gam, bet, 1e-12)
     got = stof_b200.gemm_bias_residual_layernorm(a.cuda(), w.cuda(), b.cuda(), r.cuda(), gam.cuda(), bet.cuda(), 1e-12)
     assert _err(got, want) <= 2e-3 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("m,n,k,ldc", [(9601, 256, 64, 256), (4353, 512, 200, 520), (5633, 768, 72, 784), (8065, 1024, 136, 1024), (3841, 1024, 2048, 1032)])
+def test_layernorm_epilogue_over_pairs_of_blocks(m, n, k, ldc):
+    """GEMM + LayerNorm beyond what runs at once on small tiles: clusters of 2, 4, 6 and 8 thread blocks, one to three 256-row blocks
+    each, a last one of one row, K not a multiple of the stage, row strides beyond the row, in place over the residual."""
+    import stof_b200
+    a, w, b, r = _rand((m, k), 71), _rand((k, n), 72, k ** -0.5), _rand((n,), 73), _rand((m, n), 74)
+    gam, bet = (_rand((n,), 75, 0.3).float() + 1).half(), _rand((n,), 76, 0.3)
+    want = of.gemm_bias_residual_layernorm(a, w, b, r, gam, bet, 1e-12)
+    tol = 2e-3 * max(1.0, want.abs().max().item())           # an ulp of fp16 at the largest magnitude, as above
+    buf = torch.zeros(m + 1, ldc, dtype=torch.float16, device="cuda")
+    out = buf[:m, :n]
+    out.copy_(r)
+    args = (a.cuda(), w.cuda(), b.cuda())
+    assert _err(stof_b200.gemm_bias_residual_layernorm(*args, r.cuda(), gam.cuda(), bet.cuda(), 1e-12), want) <= tol
+    stof_b200.gemm_bias_residual_layernorm(*args, out, gam.cuda(), bet.cuda(), 1e-12, out=out)
+    assert _err(out, want) <= tol
+    assert not buf[m].any() and not buf[:, n:].any()         # nothing beside the matrix is written
+    want = of.gemm_bias_residual_layernorm(a, w, torch.zeros_like(b), torch.zeros_like(r), torch.ones_like(gam), torch.zeros_like(bet), 1e-5)
+    assert _err(stof_b200.gemm_bias_residual_layernorm(args[0], args[1], None, None, None, None, 1e-5), want) <= tol
