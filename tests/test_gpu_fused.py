@@ -352,3 +352,22 @@ def test_layernorm_epilogue_over_pairs_of_blocks(m, n, k, ldc):
     assert not buf[m].any() and not buf[:, n:].any()         # nothing beside the matrix is written
     want = of.gemm_bias_residual_layernorm(a, w, torch.zeros_like(b), torch.zeros_like(r), torch.ones_like(gam), torch.zeros_like(bet), 1e-5)
     assert _err(stof_b200.gemm_bias_residual_layernorm(args[0], args[1], None, None, None, None, 1e-5), want) <= tol
+
+
+@pytest.mark.parametrize("rows,hidden", [(4735, 256), (4737, 72), (4801, 264), (9473, 768), (4737, 776), (9999, 1024)])
+def test_layernorm_two_rows_at_a_time(rows, hidden):
+    """Row counts about the line from which a warp takes two rows at a time, odd ones among them, rows that end inside a lane's chunk,
+    padded row strides, in place."""
+    import stof_b200
+    x, bias, gamma, beta = _rand((rows, hidden), 81), _rand((hidden,), 82), (_rand((hidden,), 83, 0.3).float() + 1).half(), _rand((hidden,), 84, 0.3)
+    want = of.bias_layernorm(x, bias, gamma, beta)
+    tol = 2e-3 * max(1.0, want.abs().max().item())           # an ulp of fp16 at the largest magnitude
+    assert _err(stof_b200.bias_residual_layernorm(x.cuda(), bias.cuda(), None, gamma.cuda(), beta.cuda()), want) <= tol
+    buf = torch.zeros(rows + 1, hidden + 8, dtype=torch.float16, device="cuda")
+    buf[:rows, :hidden] = x.cuda()
+    view = buf[:rows, :hidden]
+    stof_b200.bias_residual_layernorm(view, bias.cuda(), None, gamma.cuda(), beta.cuda(), out=view)
+    assert _err(view, want) <= tol
+    assert not buf[rows].any() and not buf[:, hidden:].any()
+    plain = torch.nn.functional.layer_norm(x.float(), (hidden,))
+    assert _err(stof_b200.bias_residual_layernorm(x.cuda()), plain) <= tol
