@@ -336,7 +336,7 @@ extern "C" int stof_bias_residual_layernorm(const void* x, long long ldx, const 
         return STOF_OK;
     };
     // Two rows at a time where each of the 16 warps that an SM holds gets at least that many, and no residual row doubles the ring
-    // (5120 rows of 768: 6.2 us, one at a time 6.7)
+    // (8192 rows of 768: 9.5 us one at a time, 8.0 in pairs)
     if (residual == nullptr && hidden <= 1024 && rows >= sm_count() * 2 * LN_WARPS * 2) {
         if (hidden <= 256) return launch(layernorm_kernel<1, 2>, 2, ring_smem(2));
         if (hidden <= 512) return launch(layernorm_kernel<2, 2>, 2, ring_smem(2));
