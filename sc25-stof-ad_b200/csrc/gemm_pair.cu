@@ -11,6 +11,8 @@
 //               once on its own "stage free" ("accumulator full") barrier and once on its peer's, by mapped address
 //   warps 0-7   epilogue (both blocks), same as the one-block kernel; the peer's warps report "accumulator drained" to the
 //               leader's barrier with remote mbarrier arrives
+//               (released at block scope: at cluster scope the arrive waited for the warp's earlier stores and held the next tile's
+//               products back; K = 768, 16384 rows: 2304 columns 47.8 -> 44.2 us, 3072 with GELU 70.8 -> 63.6 us)
 // Every copy and every commit names exactly one block's barrier.  Both blocks meet at a cluster barrier before they leave, so
 // that neither frees shared or tensor memory its peer may still signal, read or write.
 #include <atomic>
@@ -173,7 +175,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         __syncwarp();
                         if (lane == 0) {
                             if (leader) mbar_arrive(&bars[PB_TEMPTY + acc]);
-                            else remote_arrive(map_to_rank(smem_u32(&bars[PB_TEMPTY + acc]), 0));
+                            else remote_arrive_cta(map_to_rank(smem_u32(&bars[PB_TEMPTY + acc]), 0));
                         }
                     }
                     const int col0 = colbase + ch * 64;
