@@ -612,6 +612,10 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
         s.bn = long_arg(a[12]);
         s.heads = long_arg(a[13]);
         s.eps = double_arg(a[14]);
+        // the heads' views of qkv and ctx are made from D = hidden / heads below
+        const int64_t hid = hidden.size(2);
+        if (s.heads <= 0 || hid % s.heads != 0)
+            fail("encoder: hidden size %lld is not a multiple of the %lld heads", static_cast<long long>(hid), static_cast<long long>(s.heads));
         const int act = static_cast<int>(long_arg(a[15]));
         const bool fuse = PyObject_IsTrue(a[16]) == 1, decoder = PyObject_IsTrue(a[17]) == 1;
         const Launch l(hidden);

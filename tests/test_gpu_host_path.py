@@ -1,0 +1,30 @@
+"""What the native host path refuses, accepts and remembers, against what the operators promise."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(shape, seed, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).half()
+
+
+def _encoder(hid, heads, ffn, S, block=32, without=()):
+    """One layer with random weights (None for the names in `without`) on an all-ones mask."""
+    import stof_b200
+    shapes = {"Wqkv": (hid, 3 * hid), "bqkv": (3 * hid,), "Wo": (hid, hid), "bo": (hid,), "g1": (hid,), "b1": (hid,), "W1": (hid, ffn), "bi1": (ffn,),
+              "W2": (ffn, hid), "bi2": (hid,), "g2": (hid,), "b2": (hid,)}
+    w = {k: None if k in without else _rand(s, 90 + i, 0.1).cuda() for i, (k, s) in enumerate(shapes.items())}
+    enc = stof_b200.BertEncoder([stof_b200.EncoderWeights(**w)], heads, 1e-12, block_m=block, block_n=block)
+    enc.set_mask(torch.ones(1, S, S, dtype=torch.float16, device="cuda"))
+    return enc
+
+
+@pytest.mark.parametrize("hid,heads", [(776, 12), (1032, 16), (128, 0), (128, -2)])
+def test_stack_refuses_a_hidden_size_that_its_heads_do_not_divide(hid, heads):
+    """776 / 12 and 1032 / 16 leave a head size of 64, which every later check takes, and columns that no head computes."""
+    import stof_b200
+    with pytest.raises(stof_b200.StofError, match="heads"):
+        _encoder(hid, heads, 64, 64)(_rand((1, 64, hid), 1).cuda())
