@@ -331,6 +331,11 @@ struct Index {
 };
 
 PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads, int64_t bm, int64_t bn, int64_t dev) {
+    // On every call, known index or not: base[:n] and base[::2] of one tensor agree in all that the key holds
+    for (int i = 0; i < 4; ++i)
+        if (ix.t[i]->scalar_type() != at::kInt || !ix.t[i]->is_contiguous()) fail("block attention: index tensors must be contiguous int32");
+    if (ix.t[0]->numel() != seq / bm + 1 || ix.t[2]->numel() != seq / bm + 1)
+        fail("block attention: row pointer arrays must have S / BLOCK_M + 1 entries");
     PlanKey key;
     bool keyed = true;
     for (int i = 0; i < 4; ++i) {
@@ -347,10 +352,6 @@ PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads
                 if (i > 0) std::swap(all[i], all[0]);
                 return all[0];
             }
-    for (int i = 0; i < 4; ++i)
-        if (ix.t[i]->scalar_type() != at::kInt || !ix.t[i]->is_contiguous()) fail("block attention: index tensors must be contiguous int32");
-    if (key.numel[0] != seq / bm + 1 || key.numel[2] != seq / bm + 1)
-        fail("block attention: row pointer arrays must have S / BLOCK_M + 1 entries");
     PyObject* r = PyObject_CallFunction(g_plan_for_call, "OOOOLLLLL", ix.o[0], ix.o[1], ix.o[2], ix.o[3], static_cast<long long>(seq),
                                         static_cast<long long>(batch), static_cast<long long>(heads), static_cast<long long>(bm),
                                         static_cast<long long>(bn));

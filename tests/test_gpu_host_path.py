@@ -28,3 +28,27 @@ def test_stack_refuses_a_hidden_size_that_its_heads_do_not_divide(hid, heads):
     import stof_b200
     with pytest.raises(stof_b200.StofError, match="heads"):
         _encoder(hid, heads, 64, 64)(_rand((1, 64, hid), 1).cuda())
+
+
+def _index(S, block, band):
+    import stof_b200
+    from oracle import masks as om
+    return stof_b200.get_sparse_storage(torch.from_numpy(om.generate_sliding_mask(1, S, band, False, np.float16)).cuda(), block, block)[1:]
+
+
+def test_index_checks_hold_for_an_index_whose_plan_is_known():
+    """A strided view and a view of another type with the address, version and length of an index that has been used: refused, not
+    answered with the plan of the other."""
+    import stof_b200
+    S, block = 256, 32
+    frp, fci, prp, pci, pbm, lrp, lci = _index(S, block, 40)
+    q, k, v = (_rand((1, 2, S, 64), i).cuda() for i in range(3))
+    base = torch.zeros(2 * prp.numel(), dtype=torch.int32, device="cuda")
+    base[:prp.numel()] = prp
+    plain, strided = base[:prp.numel()], base[::2]
+    assert (plain.data_ptr(), plain._version, plain.numel()) == (strided.data_ptr(), strided._version, strided.numel())
+    for _ in range(3):                                   # decided, and remembered by the native side, at the second use
+        stof_b200.block_attention(q, k, v, torch.empty_like(q), frp, fci, plain, pci, pbm, lrp, lci, block, block)
+    for other in (strided, plain.view(torch.float32)):
+        with pytest.raises(stof_b200.StofError, match="contiguous int32"):
+            stof_b200.block_attention(q, k, v, torch.empty_like(q), frp, fci, other, pci, pbm, lrp, lci, block, block)
