@@ -275,6 +275,11 @@ bool takes_pairs(int m, int n, int k, int epilogue) {
     const bool short_residual = epilogue == STOF_EPI_BIAS_RESIDUAL && k <= 1024;
     return tiles256 >= (short_residual ? 16LL : 2LL) * pairs;
 }
+
+bool overlap(const void* p, long long p_bytes, const void* q, long long q_bytes) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+    return a < b + static_cast<uintptr_t>(q_bytes) && b < a + static_cast<uintptr_t>(p_bytes);
+}
 }  // namespace
 
 // Tiles of 256 columns that the busiest multiprocessor (or pair) walks in the GEMM kernel that a shape gets, small tiles apart
@@ -322,11 +327,15 @@ extern "C" int stof_gemm_bias_act(const void* a, long long lda, const void* w, l
         // Measured, weights from HBM, this kernel against the 128 x 256 one: K = 768: 128 rows x 768 columns 64 x 64 3.4 / 9.1 us,
         // 512 x 2304 128 x 64 5.3 / 8.9, 1000 x 2304 128 x 128 7.3 / 9.0, 512 x 3072 128 x 128 7.8 / 10.5; K = 3072, 768 columns:
         // 128 rows 64 x 64 in two parts 5.8 / 22.9, 512 rows 64 x 64 8.2 / 21.4, 1000 rows 128 x 64 10.3 / 21.1.
+        // C over A is sound where one block reads a row of A and writes it, after its last product: with tiles as wide as the matrix.
+        // (Up to 256 columns the kernel below has such tiles.)
+        const bool over_a = overlap(a, ((m - 1LL) * lda + k) * 2, c, ((m - 1LL) * ldc + n) * 2);
         const int sms = sm_count();
         constexpr int SHAPES[3][2] = {{64, 64}, {128, 64}, {128, 128}};
         for (const auto& t : SHAPES) {
             const long long tiles = static_cast<long long>((m + t[0] - 1) / t[0]) * ((n + t[1] - 1) / t[1]);
             if (tiles > sms) continue;
+            if (over_a && n > t[1]) continue;
             int split = 1;
             if (k >= 2048 && 2 * tiles <= sms) split = 2;
             if (k >= 4096 && 4 * tiles <= sms) split = 4;

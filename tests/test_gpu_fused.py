@@ -371,3 +371,22 @@ def test_layernorm_two_rows_at_a_time(rows, hidden):
     assert not buf[rows].any() and not buf[:, hidden:].any()
     plain = torch.nn.functional.layer_norm(x.float(), (hidden,))
     assert _err(stof_b200.bias_residual_layernorm(x.cuda()), plain) <= tol
+
+
+@pytest.mark.parametrize("m,n", [(1000, 64), (129, 72), (700, 128), (513, 192), (2048, 256)])
+def test_gemm_written_over_its_input(m, n):
+    """out = a, up to the 256 columns of one tile: a row of A is read by the block that writes it, and by no other."""
+    import stof_b200
+    a, w, b, r = _rand((m, n), 91), _rand((n, n), 92, n ** -0.5), _rand((n,), 93), _rand((m, n), 94)
+    base = of.gemm_bias(a, w, b)
+    tol = 2e-3 * max(1.0, base.abs().max().item())
+    wd, bd, rd = w.cuda(), b.cuda(), r.cuda()
+    for _ in range(3):
+        x = a.cuda()
+        assert stof_b200.gemm_bias(x, wd, bd, out=x) is x and _err(x, base) <= tol
+        x = a.cuda()
+        assert _err(stof_b200.gemm_bias_residual(x, wd, bd, rd, out=x), base + r.float()) <= 2 * tol
+        x = a.cuda()
+        want = of.gemm_bias_residual_layernorm(a, w, b, r, torch.ones(n).half(), torch.zeros(n).half(), 1e-5)
+        # the sums are rounded to fp16 before the LayerNorm where n is not a multiple of 256: an ulp at their largest, over their spread
+        assert _err(stof_b200.gemm_bias_residual_layernorm(x, wd, bd, rd, None, None, 1e-5, out=x), want) <= 4e-3 * max(1.0, want.abs().max().item())
