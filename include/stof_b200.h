@@ -219,8 +219,9 @@ int stof_gemm_bias_act(const void* a, long long lda, const void* w, long long ld
  *           GEMM kernel), and matmul + bias + residual + F.layer_norm of src/benchmk_end2end.py:73-76, 83-86.
  * bias, residual, gamma, beta may be NULL (0 / 0 / 1 / 0).  For n a multiple of 256 up to 1024 and k <= 2048
  * this is ONE kernel (the thread blocks of a row block - n / 256 of them, or n / 64 or n / 128 at few rows - form a
- * cluster and exchange row statistics through distributed shared memory); other shapes run stof_gemm_bias_act followed by
- * stof_bias_residual_layernorm in place (for long contractions that is the faster of the two, measured).
+ * cluster and exchange row statistics through distributed shared memory); other n run stof_gemm_bias_act followed by
+ * stof_bias_residual_layernorm in place, and so do longer contractions where that is the faster of the two, measured.  (Those
+ * round the sums to fp16 before the statistics.)
  * ------------------------------------------------------------------------------------------ */
 int stof_gemm_bias_residual_layernorm(const void* a, long long lda, const void* w, long long ldw, const void* bias,
                                       const void* residual, long long ldr, const void* gamma, const void* beta, float eps,

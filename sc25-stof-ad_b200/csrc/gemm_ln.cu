@@ -354,13 +354,15 @@ int resident_clusters(int slices, int* clusters) {
     return STOF_OK;
 }
 
-// Is one kernel faster than the GEMM followed by the LayerNorm kernel?  It saves the LayerNorm pass, but its clusters leave 13 to 28
-// SMs idle and its rounds are of whole row blocks.  A 256 x 256 tile of a pair of blocks and a 128 x 256 tile of one block take the
-// same time per 64 of K, 0.4 us; a LayerNorm pass takes that long per 300,000 elements.  Measured with residual, one kernel / two:
-// K = 3072, N = 768: 4096 rows 27.3 / 28.8 us (1 round / 1), 6144 44.1 / 31.9 (2 / 1), 8192 45.4 / 48.6 (2 / 2), 32768 134 / 142 (6 / 6);
-// K = 4096, N = 1024: 2816 rows 32.6 / 33.2 (1 / 1), 8192 79.4 / 65.8 (3 / 2), 32768 237 / 225 (9 / 7); K = N = 1024: 4096 rows 19.8 / 19.1
-// (2 / 1), 8192 27.2 / 29.9 (3 / 2), 32768 78 / 92 (9 / 7).  Where the GEMM alone would run on small tiles it stays ahead: K = 3072,
-// N = 768: 3072 rows 26.6 / 21.8; K = N = 1024: 2048 rows 14.2 / 12.4.
+// Beyond K = 2048: is one kernel faster than the GEMM followed by the LayerNorm kernel?  It saves the LayerNorm pass, but clusters of 6
+// and 8 blocks leave 16 and 28 SMs idle and its rounds are of whole row blocks.  A 256 x 256 tile of a pair of blocks and a 128 x 256
+// tile of one block take the same time per 64 of K, 0.4 us; a LayerNorm pass takes that long per 300,000 elements.  Measured with
+// residual, one kernel / two: K = 3072, N = 768: 4096 rows 27.3 / 28.8 us (1 round / 1), 6144 44.1 / 31.9 (2 / 1), 8192 45.4 / 48.6
+// (2 / 2), 32768 134 / 142 (6 / 6); K = 4096, N = 1024: 2816 rows 32.6 / 33.2 (1 / 1), 8192 79.4 / 65.8 (3 / 2), 32768 237 / 225 (9 / 7).
+// Where the GEMM alone would run on small tiles it stays ahead: K = 3072, N = 768: 3072 rows 26.6 / 21.8.
+// Up to K = 2048 it is one kernel whatever the time: two kernels round the sums to fp16 before the statistics, and rows with a common
+// offset of 60 and a spread of 0.5 then come out 3.7e-2 off, against 2e-3 (K = N = 1024: 2048 rows 14.2 us against 12.4, 4096 rows 19.8
+// against 19.1).  Beyond, two kernels have been the form of these shapes from the start.
 bool one_kernel_wins(int m, int n, int k, bool residual, int clusters) {
     if (((m + 127LL) / 128) * ((n + 127LL) / 128) <= sm_count()) return false;
     const long long rounds = ((m + 255LL) / 256 + clusters - 1) / clusters;
@@ -373,8 +375,8 @@ bool one_kernel_wins(int m, int n, int k, bool residual, int clusters) {
 
 using namespace stof;
 
-// Declared in include/stof_b200.h.  Shapes that neither fused kernel covers (N not a multiple of 256, or beyond 1024) or is faster
-// for run as the GEMM with the bias + residual epilogue followed by the row LayerNorm kernel in place.
+// Declared in include/stof_b200.h.  Shapes that neither fused kernel covers (N not a multiple of 256, or beyond 1024), and those beyond
+// K = 2048 that two kernels are faster for, run as the GEMM with the bias + residual epilogue followed by the row LayerNorm kernel in place.
 // STOF_B200_GEMM_LN=fused / split overrides.
 extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, const void* w, long long ldw, const void* bias,
                                                  const void* residual, long long ldr, const void* gamma, const void* beta, float eps,
@@ -402,7 +404,7 @@ extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, c
         const uint32_t box[2] = {64, L_BK};
         if (int rc = make_tensor_map_f16(&mw, w, 2, dims, strides, box)) return rc;
     }
-    // few rows; from K = 2048 on a row block's few thread blocks walk K longer than the split GEMM and a LayerNorm pass take
+    // few rows; beyond K = 2048 a row block's few thread blocks walk K longer than the split GEMM and a LayerNorm pass take
     if (covered && mode == 0 && k <= 2048) {
         int done = 0;
         const int rc = gemm_split_ln_dispatch({a, lda, &mw, static_cast<const __half*>(bias), static_cast<const __half*>(residual), ldr,
@@ -414,7 +416,7 @@ extern "C" int stof_gemm_bias_residual_layernorm(const void* a, long long lda, c
     if (covered)
         if (int rc = resident_clusters(slices, &clusters)) return rc;
     // (over A itself only in one kernel: nothing is written before all blocks of a row block have multiplied)
-    if (!covered || (mode != 1 && a != c && !one_kernel_wins(m, n, k, residual != nullptr, clusters))) {
+    if (!covered || (mode != 1 && k > 2048 && a != c && !one_kernel_wins(m, n, k, residual != nullptr, clusters))) {
         int rc = residual ? stof_gemm_bias_act(a, lda, w, ldw, bias, residual, ldr, c, ldc, m, n, k, STOF_EPI_BIAS_RESIDUAL, status_dev, stream_)
                           : stof_gemm_bias_act(a, lda, w, ldw, bias, nullptr, 0, c, ldc, m, n, k, STOF_EPI_BIAS, status_dev, stream_);
         if (rc != STOF_OK) return rc;

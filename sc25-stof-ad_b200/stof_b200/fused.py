@@ -53,7 +53,7 @@ def gemm_bias_residual_layernorm(a, w, bias, residual, gamma, beta, eps: float, 
     """LayerNorm(a @ w + bias + residual) * gamma + beta (src/benchmk_end2end.py:73-76, 83-86; the statistics inside the GEMM
     kernel as in src/triton_template/gemm_add_layernorm.py:77-123): for N a multiple of 256 up to 1024 and K <= 2048 ONE tcgen05
     kernel whose epilogue takes the row statistics across a cluster of thread blocks (`stof_gemm_bias_residual_layernorm`); other
-    shapes run the GEMM with the bias + residual epilogue and the LayerNorm kernel in place, behind the same entry point.
+    N, and longer K where that is faster, run the GEMM with the bias + residual epilogue and the LayerNorm kernel in place.
     bias, residual, gamma, beta may be None."""
     return (_lib._native or _lib.native()).gemm_ln(a, w, bias, residual, gamma, beta, eps, out)
 

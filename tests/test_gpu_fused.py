@@ -390,3 +390,17 @@ def test_gemm_written_over_its_input(m, n):
         want = of.gemm_bias_residual_layernorm(a, w, b, r, torch.ones(n).half(), torch.zeros(n).half(), 1e-5)
         # the sums are rounded to fp16 before the LayerNorm where n is not a multiple of 256: an ulp at their largest, over their spread
         assert _err(stof_b200.gemm_bias_residual_layernorm(x, wd, bd, rd, None, None, 1e-5, out=x), want) <= 4e-3 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("m,n,k", [(2048, 1024, 64), (4096, 1024, 64), (2100, 1024, 1024), (4500, 512, 512), (3000, 768, 768), (8000, 1024, 2048)])
+def test_layernorm_epilogue_keeps_its_sums_in_fp32_at_every_row_count(m, n, k):
+    """The large common offset again, at row counts where a GEMM and a LayerNorm kernel would be the faster form: between its two kernels
+    the sums would be rounded to fp16, 0.016 to 0.03 at 60, which a spread of 0.5 doubles."""
+    import stof_b200
+    if os.environ.get("STOF_B200_GEMM_LN", "").startswith("s"):
+        pytest.skip("this case is about the fused form")
+    a, w = _rand((m, k), 41, 0.1), _rand((k, n), 42, 0.8 * k ** -0.5)
+    r = (_rand((m, n), 43, 0.5).float() + 60.0).half()
+    got = stof_b200.gemm_bias_residual_layernorm(a.cuda(), w.cuda(), None, r.cuda(), None, None, 1e-12)
+    want = of.gemm_bias_residual_layernorm(a, w, torch.zeros(n).half(), r, torch.ones(n).half(), torch.zeros(n).half(), 1e-12)
+    assert _err(got, want) <= 4e-3
