@@ -8,7 +8,7 @@ positional arguments, and the returned tensor IS `q`, overwritten with the atten
 version raises.
 """
 import torch
-from torch.autograd import Function
+from torch.autograd import Function, forward_ad
 
 from stof_b200.attention import block_attn_mask as _block_attn_mask_forward
 from stof_b200 import rowwise as _rowwise
@@ -58,9 +58,10 @@ class Block_Attn_Mask(Function):
 
 
 # The operators are forward-only: with nothing to differentiate the autograd.Function machinery (some 10 us a call) has no effect,
-# and the call goes straight to the implementation.
+# and the call goes straight to the implementation.  Inside a forward-mode level it does not: a dual tensor does not require grad, and
+# the Function is what refuses its tangent.
 def _differentiating(q, k, v):
-    return torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
+    return forward_ad._current_level >= 0 or (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))
 
 
 def rowwise_attn_full_op(q, k, v, is_causal=False):
