@@ -45,7 +45,7 @@ const char* stof_last_error(void);
  *      {n_full, n_part, n_load, nnz_elements}.
  *   2. stof_mask_fill      : writes the column indices (ascending inside a row, `load` = merge of
  *      full and partial) and gathers the partial tiles as -10000 * (1 - m) in fp16.
- * `workspace` is scratch shared by both phases (size from stof_mask_workspace_bytes) and must stay
+ * `workspace` is scratch shared by both phases (size from stof_mask_workspace_bytes, 4-byte aligned) and must stay
  * untouched between them.  mask_dtype is STOF_DTYPE_F16 or STOF_DTYPE_F32; the mask is a dense
  * row-major (batch, S, S) array; S must be a multiple of block_m and of block_n, block_n a multiple
  * of 8.  Index outputs are int32.
@@ -66,7 +66,7 @@ int stof_mask_fill(const void* mask, int mask_dtype, int seq_len, int block_m, i
  * host).  The kernel itself writes them, with the status word, into `notice` - host memory the device can write (pinned and
  * mapped) - and last of all `stamp`, which the host polls for: nothing is copied and the stream is not synchronised.
  * `nnz_percent` (device) receives 100 * non-zeros / S^2 in fp32.  `header`: 16 bytes of device memory, zero before the first
- * call, left at zero by every call; calls that may run at the same time need headers of their own.  `workspace` as above (its
+ * call, left at zero by every call; calls that may run at the same time need headers of their own.  `workspace` as above but 16-byte aligned, like `header` (its
  * header part is not used); phase 2 is stof_mask_fill. */
 typedef struct stof_mask_notice {
     int n_full, n_part;

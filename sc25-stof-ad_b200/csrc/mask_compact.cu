@@ -37,10 +37,13 @@ constexpr int CLASSIFY_THREADS = 256;
 constexpr int MAX_TILES_PER_ROW = 4096;
 constexpr int FILL_THREADS = 256;
 
-struct Workspace {            // header at the start of the caller's workspace, class bytes follow
-    unsigned int ticket;      // blocks that finished phase 1 (reset by the last one)
-    unsigned int pad;
-    unsigned long long nnz;   // non-zero elements seen so far (read and reset by the last block)
+// Header of 16 bytes at the start of the caller's workspace, class bytes follow.  A workspace is 4-byte aligned, no more: the 64-bit
+// count lies at the multiple of 8 behind the ticket.
+struct Workspace {
+    unsigned int* ticket;     // blocks that finished phase 1 (reset by the last one)
+    unsigned long long* nnz;  // non-zero elements seen so far (read and reset by the last block)
+    explicit Workspace(void* header)
+        : ticket(static_cast<unsigned int*>(header)), nnz(reinterpret_cast<unsigned long long*>((reinterpret_cast<uintptr_t>(header) + 11) & ~uintptr_t{7})) {}
 };
 constexpr size_t WS_HEADER = 16;
 
@@ -89,7 +92,7 @@ __device__ void scan_rows(const unsigned char* cls, int nbm, int nbn, int* full_
         __syncthreads();
         const int rows_here = min(chunk, nbm - r0);
         const int cells = rows_here * nbn;
-        if ((nbn & 15) == 0) {
+        if ((nbn & 15) == 0 && (reinterpret_cast<uintptr_t>(cls) & 15) == 0) {
             // sixteen class bytes of one row at a time; bit 0 of a byte says full, bit 1 partial
             for (int i = threadIdx.x; i < cells / 16; i += blockDim.x) {
                 const uint4 v = __ldcg(reinterpret_cast<const uint4*>(cls + static_cast<size_t>(r0) * nbn) + i);
@@ -168,7 +171,7 @@ constexpr int CLASSIFY_FLIGHT = 8;            // independent 16-byte loads of a 
 template <bool F32>
 __global__ void __launch_bounds__(CLASSIFY_THREADS)
 classify_kernel(const void* __restrict__ mask, const Geometry geo, int* full_row_ptr, int* part_row_ptr, int* load_row_ptr, const Report report,
-                Workspace* ws, unsigned char* cls) {
+                const Workspace ws, unsigned char* cls) {
     constexpr int EPC = F32 ? 4 : 8;                       // elements per 16-byte chunk
     constexpr unsigned ONE = F32 ? 0x3F800000u : 0x3C003C00u, MAG = F32 ? 0x7FFFFFFFu : 0x7FFF7FFFu;
     __shared__ unsigned s_flags[CLASSIFY_THREADS];         // per tile of the stripe: 1 = some element is not 1, 2 = some element is not 0
@@ -239,21 +242,21 @@ classify_kernel(const void* __restrict__ mask, const Geometry geo, int* full_row
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
         for (int i = 0; i < CLASSIFY_THREADS / 32; ++i) t += s_nz[i];
-        if (t) atomicAdd(&ws->nnz, t);
+        if (t) atomicAdd(ws.nnz, t);
     }
     // last block of the whole grid builds the row pointers
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(&ws->ticket, 1u);
+        const unsigned t = atomicAdd(ws.ticket, 1u);
         s_last = (t == gridDim.x - 1);
-        if (s_last) ws->ticket = 0;                        // ready for the next call
+        if (s_last) *ws.ticket = 0;                        // ready for the next call
     }
     __syncthreads();
     if (s_last) {
         __threadfence();
         unsigned long long nnz = 0;
-        if (threadIdx.x == 0) nnz = atomicExch(&ws->nnz, 0ull);
+        if (threadIdx.x == 0) nnz = atomicExch(ws.nnz, 0ull);
         scan_rows(cls, nbm, nbn, full_row_ptr, part_row_ptr, load_row_ptr, report, nnz, s_rows);
     }
 }
@@ -436,7 +439,7 @@ int check_geometry(int seq_len, int bm, int bn) {
 }
 
 int launch_classify(const void* mask, int mask_dtype, int batch, int seq_len, int bm, int bn, int* full_row_ptr, int* part_row_ptr, int* load_row_ptr,
-                    const Report& report, Workspace* ws, unsigned char* cls, cudaStream_t stream) {
+                    const Report& report, const Workspace& ws, unsigned char* cls, cudaStream_t stream) {
     const bool f32 = mask_dtype == STOF_DTYPE_F32;
     const int epc = f32 ? 4 : 8;
     // Stripes of whole tiles, 512 bytes of a row or more (coalescing, few blocks), at most one 16-byte chunk per thread of a row
@@ -481,16 +484,16 @@ extern "C" int stof_mask_classify(const void* mask, int mask_dtype, int batch, i
     STOF_REQUIRE(mask_dtype == STOF_DTYPE_F16 || mask_dtype == STOF_DTYPE_F32, "mask_classify: mask_dtype must be f16 or f32");
     STOF_REQUIRE(batch >= 1 && batch <= 65535, "mask_classify: batch %d out of range", batch);
     STOF_REQUIRE(aligned16(mask), "mask_classify: mask must be 16-byte aligned");
+    STOF_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 3u) == 0, "mask_classify: workspace must be 4-byte aligned");
     if (workspace_bytes < stof_mask_workspace_bytes(seq_len, block_m, block_n)) {
         set_error("mask_classify: workspace of %zu bytes, need %zu", workspace_bytes, stof_mask_workspace_bytes(seq_len, block_m, block_n));
         return STOF_E_WORKSPACE;
     }
     const int nbm = seq_len / block_m;
     STOF_REQUIRE(nbm <= 65535, "mask_classify: more than 65535 block rows");
-    Workspace* ws = static_cast<Workspace*>(workspace);
-    STOF_CUDA(cudaMemsetAsync(ws, 0, WS_HEADER, stream));
+    STOF_CUDA(cudaMemsetAsync(workspace, 0, WS_HEADER, stream));
     const Report report{reinterpret_cast<unsigned long long*>(counts), nullptr, 0.f, nullptr, nullptr, 0};
-    return launch_classify(mask, mask_dtype, batch, seq_len, block_m, block_n, full_row_ptr, part_row_ptr, load_row_ptr, report, ws,
+    return launch_classify(mask, mask_dtype, batch, seq_len, block_m, block_n, full_row_ptr, part_row_ptr, load_row_ptr, report, Workspace(workspace),
                            static_cast<unsigned char*>(workspace) + WS_HEADER, stream);
 }
 
@@ -510,7 +513,7 @@ extern "C" int stof_mask_classify_notify(const void* mask, int mask_dtype, int b
     }
     const Report report{nullptr, nnz_percent, 1.0f / static_cast<float>(static_cast<long long>(seq_len) * seq_len), status_dev, notice, stamp};
     return launch_classify(mask, mask_dtype, batch, seq_len, block_m, block_n, full_row_ptr, part_row_ptr, load_row_ptr, report,
-                           static_cast<Workspace*>(header), static_cast<unsigned char*>(workspace) + WS_HEADER, stream);
+                           Workspace(header), static_cast<unsigned char*>(workspace) + WS_HEADER, stream);
 }
 
 extern "C" int stof_mask_fill(const void* mask, int mask_dtype, int seq_len, int block_m, int block_n, const int* full_row_ptr,
@@ -560,13 +563,13 @@ extern "C" int stof_mask_compact_static(const void* mask, int mask_dtype, int ba
     }
     unsigned char* scratch = nullptr;
     if (int rc = static_scratch_address(&scratch)) return rc;
-    Workspace* ws = reinterpret_cast<Workspace*>(scratch);
     unsigned char* cls = scratch + WS_HEADER;
 
     // the array keeps what the previous call left: the ticket and the count must start at zero
-    STOF_CUDA(cudaMemsetAsync(ws, 0, WS_HEADER, stream));
+    STOF_CUDA(cudaMemsetAsync(scratch, 0, WS_HEADER, stream));
     const Report report{reinterpret_cast<unsigned long long*>(counts), nullptr, 0.f, nullptr, nullptr, 0};
-    if (int rc = launch_classify(mask, mask_dtype, batch, seq_len, block_m, block_n, full_row_ptr, part_row_ptr, load_row_ptr, report, ws, cls, stream))
+    if (int rc = launch_classify(mask, mask_dtype, batch, seq_len, block_m, block_n, full_row_ptr, part_row_ptr, load_row_ptr, report, Workspace(scratch), cls,
+                                 stream))
         return rc;
     int shares = (4 * sm_count() + nbm - 1) / nbm;
     if (shares < 1) shares = 1;

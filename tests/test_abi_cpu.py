@@ -273,3 +273,16 @@ def test_host_pipeline_chunking():
         for chunk in (1, 2, 5):
             sizes = tapered_chunks(batch, chunk, 2)
             assert sum(sizes) == batch and max(sizes) <= chunk and min(sizes) >= 1
+
+
+def test_compaction_workspace_alignment(built_lib):
+    """What the kernels cannot read is refused on the host: a workspace off a multiple of 4, or of 16 where the class bytes are read
+    sixteen at a time whatever the address."""
+    L, _ = built_lib
+    at = lambda a: ctypes.c_void_p(a)
+    for off in (1, 2, 3):
+        rc = L.stof_mask_classify(at(256), 0, 1, 128, 64, 64, at(256), at(256), at(256), at(256), at(256 + off), 1 << 20, None)
+        assert rc == -1 and b"aligned" in L.stof_last_error()
+    for ws, header in ((260, 256), (256, 264)):
+        rc = L.stof_mask_classify_notify(at(256), 0, 1, 128, 64, 64, at(256), at(256), at(256), at(256), at(ws), 1 << 20, at(header), None, at(256), 1, None)
+        assert rc == -1 and b"aligned" in L.stof_last_error()

@@ -130,3 +130,30 @@ def test_compaction_stripe_and_tile_edges(seq_len, bm, bn, batch, dtype):
     got, st = _run(mask, bm, bn), om.get_sparse_storage(mask, bm, bn)
     share = torch.tensor(np.count_nonzero(mask), device="cuda") / (seq_len * seq_len) * 100        # the same fp32 operations on the GPU
     _compare(got, dataclasses.replace(st, nnz=share.item()))
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8, 12])
+def test_compaction_in_a_workspace_at_any_multiple_of_four(offset):
+    """The C ABI with a workspace cut out of a larger buffer, at a number of tiles per row (16) that is read sixteen class bytes at a time."""
+    from stof_b200 import _lib
+    L, S, b = _lib.lib(), 512, 32
+    mask_np = om.generate_sliding_mask(2, S, 70, False, np.float16)
+    st, mask = om.get_sparse_storage(mask_np, b, b), torch.from_numpy(mask_np).cuda()
+    n = int(L.stof_mask_workspace_bytes(S, b, b))
+    buf = torch.full((n + 32,), 0xA5, dtype=torch.uint8, device="cuda")
+    ws, ptrs, counts = buf[offset:offset + n], torch.empty(3, S // b + 1, dtype=torch.int32, device="cuda"), torch.empty(4, dtype=torch.int64, device="cuda")
+    stream = _lib.current_stream_ptr(mask.device)
+    p = [_lib.ptr(x) for x in ptrs]
+    _lib.check(L.stof_mask_classify(_lib.ptr(mask), _lib.STOF_DTYPE_F16, 2, S, b, b, *p, _lib.ptr(counts), _lib.ptr(ws), n, stream), "classify")
+    n_full, n_part, n_load, nnz = counts.tolist()
+    assert (n_full, n_part, n_load, nnz) == (st.full_col_idx.size, st.part_col_idx.size, st.load_col_idx.size, int(np.count_nonzero(mask_np)))
+    cols = torch.empty(3, n_load, dtype=torch.int32, device="cuda")
+    tiles = torch.empty(n_part, b, b, dtype=torch.float16, device="cuda")
+    _lib.check(L.stof_mask_fill(_lib.ptr(mask), _lib.STOF_DTYPE_F16, S, b, b, *p, *(_lib.ptr(c) for c in cols), _lib.ptr(tiles), _lib.ptr(ws), n, stream), "fill")
+    torch.cuda.synchronize()
+    for got, want in zip(ptrs, (st.full_row_ptr, st.part_row_ptr, st.load_row_ptr)):
+        assert np.array_equal(got.cpu().numpy(), want)
+    for got, want in zip(cols, (st.full_col_idx, st.part_col_idx, st.load_col_idx)):
+        assert np.array_equal(got.cpu().numpy()[:want.size], want)
+    assert np.array_equal(tiles.cpu().numpy().view(np.uint16), st.part_block_mask.view(np.uint16))
+    assert (buf[:offset] == 0xA5).all() and (buf[offset + n:] == 0xA5).all()       # nothing beside the workspace is written
