@@ -86,7 +86,6 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(table) + L_TABLE_BYTES);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + LB_COUNT);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* peer_abort = reinterpret_cast<int*>(tmem_slot + 2);         // [2 * L_MAX_SLICES]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = static_cast<int>(cluster_rank()), size = 2 * slices;
@@ -99,7 +98,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const WaitCtx wctx{abort_flag, status};
 
     if (threadIdx.x == 0) {
-        *abort_flag = (status != nullptr && *status != 0) ? 1 : 0;
+        *abort_flag = 0;
         for (int i = 0; i < L_STAGES; ++i) {
             mbar_init(&bars[LB_FULL + i], 1);                 // the leader's: its own arrive.expect_tx; bytes from both blocks of the pair
             mbar_init(&bars[LB_EMPTY + i], 1);                // a commit of the leader, in both blocks
@@ -122,205 +121,193 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // The status word is read by every block on its own; a block that sat out while its peers ran would leave them waiting for
-    // its partials until their wait budgets ran out.  So the decision to run is taken per cluster: every block tells every
-    // peer through a flag in shared memory and all of them run only if none objects.
-    if (threadIdx.x < size) {
-        const uint32_t dst = map_to_rank(smem_u32(&peer_abort[rank]), static_cast<uint32_t>(threadIdx.x));
-        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(*abort_flag) : "memory");
-    }
-    __syncwarp();
-    cluster_sync_all();
-    bool run = true;
-    for (int i = 0; i < size; ++i) run = run && peer_abort[i] == 0;
     grid_dependency_wait();
     grid_launch_dependents();
 
-    if (run) {
-        if (warp == L_EPI_WARPS) {
-            // ------------------------------------------------------------------ TMA producer (both blocks of a pair)
-            if (elect_one()) {
-                tma_prefetch_desc(&map_a);
-                tma_prefetch_desc(&map_w);
-                int it = 0;
-                for (int rb = cluster_id; rb < tiles_m; rb += clusters) {
-                    const int m0 = rb * (2 * L_BM) + half * L_BM;
-                    const int w0 = n0 + half * (L_BN / 2);
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % L_STAGES;
-                        const uint32_t ph = (it / L_STAGES) & 1;
-                        mbar_wait(&bars[LB_EMPTY + s], ph ^ 1, wctx, LB_EMPTY + s);
-                        if (leader) mbar_arrive_expect_tx(&bars[LB_FULL + s], 2 * L_STAGE_BYTES);
-                        const uint32_t full = map_to_rank(smem_u32(&bars[LB_FULL + s]), static_cast<uint32_t>(rank & ~1));
-                        unsigned char* a_dst = smem + s * L_STAGE_BYTES;
-                        unsigned char* b_dst = a_dst + L_A_BYTES;
-                        tma_load_2d_pair(a_dst, &map_a, full, kb * L_BK, m0);
+    if (warp == L_EPI_WARPS) {
+        // ------------------------------------------------------------------ TMA producer (both blocks of a pair)
+        if (elect_one()) {
+            tma_prefetch_desc(&map_a);
+            tma_prefetch_desc(&map_w);
+            int it = 0;
+            for (int rb = cluster_id; rb < tiles_m; rb += clusters) {
+                const int m0 = rb * (2 * L_BM) + half * L_BM;
+                const int w0 = n0 + half * (L_BN / 2);
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % L_STAGES;
+                    const uint32_t ph = (it / L_STAGES) & 1;
+                    mbar_wait(&bars[LB_EMPTY + s], ph ^ 1, wctx, LB_EMPTY + s);
+                    if (leader) mbar_arrive_expect_tx(&bars[LB_FULL + s], 2 * L_STAGE_BYTES);
+                    const uint32_t full = map_to_rank(smem_u32(&bars[LB_FULL + s]), static_cast<uint32_t>(rank & ~1));
+                    unsigned char* a_dst = smem + s * L_STAGE_BYTES;
+                    unsigned char* b_dst = a_dst + L_A_BYTES;
+                    tma_load_2d_pair(a_dst, &map_a, full, kb * L_BK, m0);
 #pragma unroll
-                        for (int j = 0; j < L_BN / 128; ++j)
-                            tma_load_2d_pair(b_dst + j * (L_BK * 64 * 2), &map_w, full, w0 + 64 * j, kb * L_BK);
-                    }
+                    for (int j = 0; j < L_BN / 128; ++j)
+                        tma_load_2d_pair(b_dst + j * (L_BK * 64 * 2), &map_w, full, w0 + 64 * j, kb * L_BK);
                 }
             }
-        } else if (warp == L_EPI_WARPS + 1) {
-            // ------------------------------------------------------------------ MMA issuer (leader of a pair)
-            if (leader && elect_one()) {
-                constexpr uint32_t idesc = make_idesc_f16(2 * L_BM, L_BN, /*b_mn_major=*/true);
-                const uint32_t peer = static_cast<uint32_t>(rank + 1);
-                int it = 0, tile = 0;
-                for (int rb = cluster_id; rb < tiles_m; rb += clusters, ++tile) {
-                    const int acc = tile & 1;
-                    const uint32_t acc_ph = (tile >> 1) & 1;
-                    mbar_wait(&bars[LB_TEMPTY + acc], acc_ph ^ 1, wctx, LB_TEMPTY + acc);
-                    tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * L_BN;
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % L_STAGES;
-                        const uint32_t ph = (it / L_STAGES) & 1;
-                        mbar_wait(&bars[LB_FULL + s], ph, wctx, LB_FULL + s);
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_u32(smem + s * L_STAGE_BYTES);
-                        const uint32_t b_addr = a_addr + L_A_BYTES;
-#pragma unroll
-                        for (int kk = 0; kk < L_BK / 16; ++kk) {
-                            const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-                            const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, L_BK * 64 * 2, 1024);
-                            mma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-                        }
-                        tc_commit_pair(smem_u32(&bars[LB_EMPTY + s]));
-                        tc_commit_pair(map_to_rank(smem_u32(&bars[LB_EMPTY + s]), peer));
-                    }
-                    tc_commit_pair(smem_u32(&bars[LB_TFULL + acc]));
-                    tc_commit_pair(map_to_rank(smem_u32(&bars[LB_TFULL + acc]), peer));
-                }
-            }
-        } else {
-            // ------------------------------------------------------------------ epilogue (all blocks)
-            const int quarter = warp & 3, part = warp >> 2;
-            const int lrow = quarter * 32 + lane;                 // row inside the block's 128 = tensor-memory lane
-            const int col0 = n0 + part * 64;
-            unsigned char* slab = slabs + warp * L_SLAB_BYTES;
-            unsigned char* slab_row = slab + lane * 128;
-            uint64_t* res_bar = &bars[LB_RES + warp];
-            const float inv_n = 1.0f / static_cast<float>(n);
-            auto request_residual = [&](int rb) {                 // one lane: the warp's 32 x 64 piece, rows beyond the matrix as zeros
-                mbar_arrive_expect_tx(res_bar, L_SLAB_BYTES);
-                tma_load_2d(slab, &map_r, res_bar, col0, rb * (2 * L_BM) + half * L_BM + quarter * 32);
-            };
-            if (has_residual && lane == 0 && cluster_id < tiles_m) request_residual(cluster_id);
-            if (threadIdx.x < 3 * L_BN / 2) {                     // the block's columns of the three vectors
-                const int v = threadIdx.x / (L_BN / 2), i = threadIdx.x % (L_BN / 2);
-                const __half* src = v == 0 ? bias : (v == 1 ? gamma : beta);
-                const float none = v == 1 ? 1.0f : 0.0f;
-                reinterpret_cast<float2*>(s_vec)[threadIdx.x] =
-                    src != nullptr ? __half22float2(*reinterpret_cast<const __half2*>(src + n0 + 2 * i)) : make_float2(none, none);
-            }
-            asm volatile("bar.sync 5, %0;" ::"n"(L_EPI_WARPS * 32) : "memory");
-            const float4* v_bias = reinterpret_cast<const float4*>(s_vec) + part * 16;
-            const float4 *v_gamma = v_bias + L_BN / 4, *v_beta = v_gamma + L_BN / 4;
-            int tile = 0;
+        }
+    } else if (warp == L_EPI_WARPS + 1) {
+        // ------------------------------------------------------------------ MMA issuer (leader of a pair)
+        if (leader && elect_one()) {
+            constexpr uint32_t idesc = make_idesc_f16(2 * L_BM, L_BN, /*b_mn_major=*/true);
+            const uint32_t peer = static_cast<uint32_t>(rank + 1);
+            int it = 0, tile = 0;
             for (int rb = cluster_id; rb < tiles_m; rb += clusters, ++tile) {
                 const int acc = tile & 1;
                 const uint32_t acc_ph = (tile >> 1) & 1;
-                const int row0 = rb * (2 * L_BM) + half * L_BM + quarter * 32;
-                float2 x[32];
-                if (has_residual && lane == 0 && rb + clusters < tiles_m) tma_prefetch_2d(&map_r, col0, row0 + clusters * (2 * L_BM));
-                mbar_wait(&bars[LB_TFULL + acc], acc_ph, wctx, LB_TFULL + acc);
+                mbar_wait(&bars[LB_TEMPTY + acc], acc_ph ^ 1, wctx, LB_TEMPTY + acc);
                 tc_fence_after();
-                {
-                    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * L_BN + part * 64;
-                    uint32_t r0[32], r1[32];
-                    tmem_ld32(t_row, r0);
-                    tmem_ld32(t_row + 32, r1);
-                    tc_wait_ld();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {                              // the accumulator has been read: hand it back to the leader's MMA warp
-                        if (leader) mbar_arrive(&bars[LB_TEMPTY + acc]);
-                        else remote_arrive_cta(map_to_rank(smem_u32(&bars[LB_TEMPTY + acc]), static_cast<uint32_t>(rank - 1)));
+                const uint32_t d_tmem = tmem_base + acc * L_BN;
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % L_STAGES;
+                    const uint32_t ph = (it / L_STAGES) & 1;
+                    mbar_wait(&bars[LB_FULL + s], ph, wctx, LB_FULL + s);
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * L_STAGE_BYTES);
+                    const uint32_t b_addr = a_addr + L_A_BYTES;
+#pragma unroll
+                    for (int kk = 0; kk < L_BK / 16; ++kk) {
+                        const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
+                        const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, L_BK * 64 * 2, 1024);
+                        mma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                     }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        x[i] = pk2(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1]));
-                        x[16 + i] = pk2(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1]));
-                    }
+                    tc_commit_pair(smem_u32(&bars[LB_EMPTY + s]));
+                    tc_commit_pair(map_to_rank(smem_u32(&bars[LB_EMPTY + s]), peer));
                 }
-                if (has_residual) {
-                    mbar_wait(res_bar, static_cast<uint32_t>(tile & 1), wctx, LB_RES);
-                } else {
-                    if (lane == 0) tma_store_wait_read();         // the slab's previous store has been read out
-                    __syncwarp();
-                }
-                // x = accumulator + bias + residual; mean and centred sum of squares over this thread's 64 columns
-                float2 sum_a = pk2(0.f, 0.f), sum_b = pk2(0.f, 0.f);
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    uint4 ru = make_uint4(0u, 0u, 0u, 0u);
-                    if (has_residual) ru = *reinterpret_cast<const uint4*>(slab_row + ((g ^ (lane & 7)) << 4));
-                    const __half2* rh = reinterpret_cast<const __half2*>(&ru);
-#pragma unroll
-                    for (int j = 0; j < 4; j += 2) {
-                        const float4 b = v_bias[2 * g + j / 2];
-                        float2 &v0 = x[4 * g + j], &v1 = x[4 * g + j + 1];
-                        v0 = add2(add2(v0, pk2(b.x, b.y)), __half22float2(rh[j]));
-                        v1 = add2(add2(v1, pk2(b.z, b.w)), __half22float2(rh[j + 1]));
-                        sum_a = add2(sum_a, v0);
-                        sum_b = add2(sum_b, v1);
-                    }
-                }
-                sum_a = add2(sum_a, sum_b);
-                const float mean_p = (sum_a.x + sum_a.y) * (1.0f / 64.0f);
-                const float2 nm = pk2(-mean_p, -mean_p);
-                float2 sq_a = pk2(0.f, 0.f), sq_b = pk2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float2 da = add2(x[i], nm), db = add2(x[i + 1], nm);
-                    sq_a = fma2(da, da, sq_a);
-                    sq_b = fma2(db, db, sq_b);
-                }
-                sq_a = add2(sq_a, sq_b);
-                // the four warps of these rows merge theirs, then warp `part` brings the block's result to column slice `part`
-                float2* mine = local + acc * L_PARTS * L_BM + lrow;
-                if (threadIdx.x == 0) mbar_arrive_expect_tx(&bars[LB_PART + acc], static_cast<uint32_t>(slices * L_BM * 8));
-                mine[part * L_BM] = make_float2(mean_p, sq_a.x + sq_a.y);
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(L_PARTS * 32) : "memory");
-                if (part < slices) {
-                    const float2 t = merge_parts<64>(mine, L_PARTS);
-                    const uint32_t to = static_cast<uint32_t>(2 * part + half);
-                    st_async_f32x2(map_to_rank(smem_u32(table + (acc * L_MAX_SLICES + slice) * L_BM + lrow), to), t.x, t.y,
-                                   map_to_rank(smem_u32(&bars[LB_PART + acc]), to));
-                }
-                mbar_wait_cluster(&bars[LB_PART + acc], acc_ph, wctx, LB_PART + acc);
-                const float2 stat = merge_parts<L_BN>(table + acc * L_MAX_SLICES * L_BM + lrow, slices);
-                const float rstd = 1.0f / sqrtf(stat.y * inv_n + eps);
-                const float2 rstd2 = pk2(rstd, rstd), shift2 = pk2(-stat.x * rstd, -stat.x * rstd);
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    uint32_t o[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j += 2) {
-                        const float4 ga = v_gamma[2 * g + j / 2], be = v_beta[2 * g + j / 2];
-                        const float2 y0 = fma2(fma2(x[4 * g + j], rstd2, shift2), pk2(ga.x, ga.y), pk2(be.x, be.y));
-                        const float2 y1 = fma2(fma2(x[4 * g + j + 1], rstd2, shift2), pk2(ga.z, ga.w), pk2(be.z, be.w));
-                        o[j] = pack_half2(y0.x, y0.y);
-                        o[j + 1] = pack_half2(y1.x, y1.y);
-                    }
-                    *reinterpret_cast<uint4*>(slab_row + ((g ^ (lane & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-                fence_proxy_async_smem();
+                tc_commit_pair(smem_u32(&bars[LB_TFULL + acc]));
+                tc_commit_pair(map_to_rank(smem_u32(&bars[LB_TFULL + acc]), peer));
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue (all blocks)
+        const int quarter = warp & 3, part = warp >> 2;
+        const int lrow = quarter * 32 + lane;                 // row inside the block's 128 = tensor-memory lane
+        const int col0 = n0 + part * 64;
+        unsigned char* slab = slabs + warp * L_SLAB_BYTES;
+        unsigned char* slab_row = slab + lane * 128;
+        uint64_t* res_bar = &bars[LB_RES + warp];
+        const float inv_n = 1.0f / static_cast<float>(n);
+        const bool mute = failure_reported(status);
+        auto request_residual = [&](int rb) {                 // one lane: the warp's 32 x 64 piece, rows beyond the matrix as zeros
+            mbar_arrive_expect_tx(res_bar, L_SLAB_BYTES);
+            tma_load_2d(slab, &map_r, res_bar, col0, rb * (2 * L_BM) + half * L_BM + quarter * 32);
+        };
+        if (has_residual && lane == 0 && cluster_id < tiles_m) request_residual(cluster_id);
+        if (threadIdx.x < 3 * L_BN / 2) {                     // the block's columns of the three vectors
+            const int v = threadIdx.x / (L_BN / 2), i = threadIdx.x % (L_BN / 2);
+            const __half* src = v == 0 ? bias : (v == 1 ? gamma : beta);
+            const float none = v == 1 ? 1.0f : 0.0f;
+            reinterpret_cast<float2*>(s_vec)[threadIdx.x] =
+                src != nullptr ? __half22float2(*reinterpret_cast<const __half2*>(src + n0 + 2 * i)) : make_float2(none, none);
+        }
+        asm volatile("bar.sync 5, %0;" ::"n"(L_EPI_WARPS * 32) : "memory");
+        const float4* v_bias = reinterpret_cast<const float4*>(s_vec) + part * 16;
+        const float4 *v_gamma = v_bias + L_BN / 4, *v_beta = v_gamma + L_BN / 4;
+        int tile = 0;
+        for (int rb = cluster_id; rb < tiles_m; rb += clusters, ++tile) {
+            const int acc = tile & 1;
+            const uint32_t acc_ph = (tile >> 1) & 1;
+            const int row0 = rb * (2 * L_BM) + half * L_BM + quarter * 32;
+            float2 x[32];
+            if (has_residual && lane == 0 && rb + clusters < tiles_m) tma_prefetch_2d(&map_r, col0, row0 + clusters * (2 * L_BM));
+            mbar_wait(&bars[LB_TFULL + acc], acc_ph, wctx, LB_TFULL + acc);
+            tc_fence_after();
+            {
+                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * L_BN + part * 64;
+                uint32_t r0[32], r1[32];
+                tmem_ld32(t_row, r0);
+                tmem_ld32(t_row + 32, r1);
+                tc_wait_ld();
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    if (row0 < m) {
-                        tma_store_2d(&map_c, slab, col0, row0);           // rows beyond the matrix are clipped by the tensor map
-                        tma_store_commit();
-                    }
-                    if (has_residual && rb + clusters < tiles_m) {
-                        tma_store_wait_read();
-                        request_residual(rb + clusters);
-                    }
+                if (lane == 0) {                              // the accumulator has been read: hand it back to the leader's MMA warp
+                    if (leader) mbar_arrive(&bars[LB_TEMPTY + acc]);
+                    else remote_arrive_cta(map_to_rank(smem_u32(&bars[LB_TEMPTY + acc]), static_cast<uint32_t>(rank - 1)));
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    x[i] = pk2(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1]));
+                    x[16 + i] = pk2(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1]));
                 }
             }
-            if (lane == 0) tma_store_wait_all();
+            if (has_residual) {
+                mbar_wait(res_bar, static_cast<uint32_t>(tile & 1), wctx, LB_RES);
+            } else {
+                if (lane == 0) tma_store_wait_read();         // the slab's previous store has been read out
+                __syncwarp();
+            }
+            // x = accumulator + bias + residual; mean and centred sum of squares over this thread's 64 columns
+            float2 sum_a = pk2(0.f, 0.f), sum_b = pk2(0.f, 0.f);
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                uint4 ru = make_uint4(0u, 0u, 0u, 0u);
+                if (has_residual) ru = *reinterpret_cast<const uint4*>(slab_row + ((g ^ (lane & 7)) << 4));
+                const __half2* rh = reinterpret_cast<const __half2*>(&ru);
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    const float4 b = v_bias[2 * g + j / 2];
+                    float2 &v0 = x[4 * g + j], &v1 = x[4 * g + j + 1];
+                    v0 = add2(add2(v0, pk2(b.x, b.y)), __half22float2(rh[j]));
+                    v1 = add2(add2(v1, pk2(b.z, b.w)), __half22float2(rh[j + 1]));
+                    sum_a = add2(sum_a, v0);
+                    sum_b = add2(sum_b, v1);
+                }
+            }
+            sum_a = add2(sum_a, sum_b);
+            const float mean_p = (sum_a.x + sum_a.y) * (1.0f / 64.0f);
+            const float2 nm = pk2(-mean_p, -mean_p);
+            float2 sq_a = pk2(0.f, 0.f), sq_b = pk2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                const float2 da = add2(x[i], nm), db = add2(x[i + 1], nm);
+                sq_a = fma2(da, da, sq_a);
+                sq_b = fma2(db, db, sq_b);
+            }
+            sq_a = add2(sq_a, sq_b);
+            // the four warps of these rows merge theirs, then warp `part` brings the block's result to column slice `part`
+            float2* mine = local + acc * L_PARTS * L_BM + lrow;
+            if (threadIdx.x == 0) mbar_arrive_expect_tx(&bars[LB_PART + acc], static_cast<uint32_t>(slices * L_BM * 8));
+            mine[part * L_BM] = make_float2(mean_p, sq_a.x + sq_a.y);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(L_PARTS * 32) : "memory");
+            if (part < slices) {
+                const float2 t = merge_parts<64>(mine, L_PARTS);
+                const uint32_t to = static_cast<uint32_t>(2 * part + half);
+                st_async_f32x2(map_to_rank(smem_u32(table + (acc * L_MAX_SLICES + slice) * L_BM + lrow), to), t.x, t.y,
+                               map_to_rank(smem_u32(&bars[LB_PART + acc]), to));
+            }
+            mbar_wait_cluster(&bars[LB_PART + acc], acc_ph, wctx, LB_PART + acc);
+            const float2 stat = merge_parts<L_BN>(table + acc * L_MAX_SLICES * L_BM + lrow, slices);
+            const float rstd = 1.0f / sqrtf(stat.y * inv_n + eps);
+            const float2 rstd2 = pk2(rstd, rstd), shift2 = pk2(-stat.x * rstd, -stat.x * rstd);
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    const float4 ga = v_gamma[2 * g + j / 2], be = v_beta[2 * g + j / 2];
+                    const float2 y0 = fma2(fma2(x[4 * g + j], rstd2, shift2), pk2(ga.x, ga.y), pk2(be.x, be.y));
+                    const float2 y1 = fma2(fma2(x[4 * g + j + 1], rstd2, shift2), pk2(ga.z, ga.w), pk2(be.z, be.w));
+                    o[j] = pack_half2(y0.x, y0.y);
+                    o[j + 1] = pack_half2(y1.x, y1.y);
+                }
+                *reinterpret_cast<uint4*>(slab_row + ((g ^ (lane & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                if (row0 < m && !mute) {
+                    tma_store_2d(&map_c, slab, col0, row0);           // rows beyond the matrix are clipped by the tensor map
+                    tma_store_commit();
+                }
+                if (has_residual && rb + clusters < tiles_m) {
+                    tma_store_wait_read();
+                    request_residual(rb + clusters);
+                }
+            }
         }
+        if (lane == 0) tma_store_wait_all();
     }
     // no block leaves while a peer may still write its table, signal one of its barriers, read its shared memory or write its tensor memory
     tc_fence_before();

@@ -57,7 +57,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const WaitCtx wctx{abort_flag, status};
 
     if (threadIdx.x == 0) {
-        *abort_flag = (status != nullptr && *status != 0) ? 1 : 0;
+        *abort_flag = 0;
         for (int i = 0; i < P_STAGES; ++i) {
             mbar_init(&bars[PB_FULL + i], 1);                 // the leader's: its own arrive.expect_tx; bytes from both blocks
             mbar_init(&bars[PB_EMPTY + i], 1);                // a tcgen05.commit of the leader, in both blocks
@@ -80,164 +80,163 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     grid_dependency_wait();
     grid_launch_dependents();
 
-    if (*abort_flag == 0) {
-        if (warp == P_EPI_WARPS) {
-            // ------------------------------------------------------------------ TMA producer (both blocks)
-            if (elect_one()) {
-                tma_prefetch_desc(&map_a);
-                tma_prefetch_desc(&map_w);
-                int it = 0;
-                for (int t = pair; t < num_tiles; t += pairs) {
-                    const int m0 = (t / tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
-                    const int n0 = (t % tiles_n) * P_BN + static_cast<int>(rank) * (P_BN / 2);
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % P_STAGES;
-                        const uint32_t ph = (it / P_STAGES) & 1;
-                        mbar_wait(&bars[PB_EMPTY + s], ph ^ 1, wctx, PB_EMPTY + s);
-                        if (leader) mbar_arrive_expect_tx(&bars[PB_FULL + s], 2 * P_STAGE_BYTES);
-                        const uint32_t full = map_to_rank(smem_u32(&bars[PB_FULL + s]), 0);
-                        unsigned char* a_dst = smem + s * P_STAGE_BYTES;
-                        unsigned char* b_dst = a_dst + P_A_BYTES;
-                        tma_load_2d_pair(a_dst, &map_a, full, kb * P_BK, m0);
+    if (warp == P_EPI_WARPS) {
+        // ------------------------------------------------------------------ TMA producer (both blocks)
+        if (elect_one()) {
+            tma_prefetch_desc(&map_a);
+            tma_prefetch_desc(&map_w);
+            int it = 0;
+            for (int t = pair; t < num_tiles; t += pairs) {
+                const int m0 = (t / tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM;
+                const int n0 = (t % tiles_n) * P_BN + static_cast<int>(rank) * (P_BN / 2);
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % P_STAGES;
+                    const uint32_t ph = (it / P_STAGES) & 1;
+                    mbar_wait(&bars[PB_EMPTY + s], ph ^ 1, wctx, PB_EMPTY + s);
+                    if (leader) mbar_arrive_expect_tx(&bars[PB_FULL + s], 2 * P_STAGE_BYTES);
+                    const uint32_t full = map_to_rank(smem_u32(&bars[PB_FULL + s]), 0);
+                    unsigned char* a_dst = smem + s * P_STAGE_BYTES;
+                    unsigned char* b_dst = a_dst + P_A_BYTES;
+                    tma_load_2d_pair(a_dst, &map_a, full, kb * P_BK, m0);
 #pragma unroll
-                        for (int j = 0; j < P_BN / 128; ++j)
-                            tma_load_2d_pair(b_dst + j * (P_BK * 64 * 2), &map_w, full, n0 + 64 * j, kb * P_BK);
-                    }
+                    for (int j = 0; j < P_BN / 128; ++j)
+                        tma_load_2d_pair(b_dst + j * (P_BK * 64 * 2), &map_w, full, n0 + 64 * j, kb * P_BK);
                 }
             }
-        } else if (warp == P_EPI_WARPS + 1) {
-            // ------------------------------------------------------------------ MMA issuer (leader only)
-            if (leader && elect_one()) {
-                constexpr uint32_t idesc = make_idesc_f16(2 * P_BM, P_BN, /*b_mn_major=*/true);
-                int it = 0, local = 0;
-                for (int t = pair; t < num_tiles; t += pairs, ++local) {
-                    const int acc = local & 1;
-                    const uint32_t acc_ph = (local >> 1) & 1;
-                    mbar_wait(&bars[PB_TEMPTY + acc], acc_ph ^ 1, wctx, PB_TEMPTY + acc);
-                    tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * P_BN;
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % P_STAGES;
-                        const uint32_t ph = (it / P_STAGES) & 1;
-                        mbar_wait(&bars[PB_FULL + s], ph, wctx, PB_FULL + s);
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_u32(smem + s * P_STAGE_BYTES);
-                        const uint32_t b_addr = a_addr + P_A_BYTES;
-#pragma unroll
-                        for (int kk = 0; kk < P_BK / 16; ++kk) {
-                            const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-                            const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, P_BK * 64 * 2, 1024);
-                            mma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-                        }
-                        // the stage is free in both blocks: one commit per block's barrier
-                        tc_commit_pair(smem_u32(&bars[PB_EMPTY + s]));
-                        tc_commit_pair(map_to_rank(smem_u32(&bars[PB_EMPTY + s]), 1));
-                    }
-                    tc_commit_pair(smem_u32(&bars[PB_TFULL + acc]));
-                    tc_commit_pair(map_to_rank(smem_u32(&bars[PB_TFULL + acc]), 1));
-                }
-            }
-        } else {
-            // ------------------------------------------------------------------ epilogue (both blocks)
-            const int quarter = warp & 3, half_n = warp >> 2;
-            unsigned char* slab = slabs + warp * P_SLAB_BYTES;
-            int local = 0;
+        }
+    } else if (warp == P_EPI_WARPS + 1) {
+        // ------------------------------------------------------------------ MMA issuer (leader only)
+        if (leader && elect_one()) {
+            constexpr uint32_t idesc = make_idesc_f16(2 * P_BM, P_BN, /*b_mn_major=*/true);
+            int it = 0, local = 0;
             for (int t = pair; t < num_tiles; t += pairs, ++local) {
                 const int acc = local & 1;
                 const uint32_t acc_ph = (local >> 1) & 1;
-                const int m0 = (t / tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM, n0 = (t % tiles_n) * P_BN;
-                const int row0 = m0 + quarter * 32;
-                const int row = row0 + lane;
-                const int colbase = n0 + half_n * (P_BN / 2);
-                uint4 res[2][8];
-                if (EPI == STOF_EPI_BIAS_RESIDUAL) {
-#pragma unroll
-                    for (int ch = 0; ch < 2; ++ch)
-#pragma unroll
-                        for (int g = 0; g < 8; ++g) {
-                            const int col = colbase + ch * 64 + g * 8;
-                            res[ch][g] = (row < m && col < n) ? __ldg(reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * ldr + col))
-                                                              : make_uint4(0u, 0u, 0u, 0u);
-                        }
-                }
-                mbar_wait(&bars[PB_TFULL + acc], acc_ph, wctx, PB_TFULL + acc);
+                mbar_wait(&bars[PB_TEMPTY + acc], acc_ph ^ 1, wctx, PB_TEMPTY + acc);
                 tc_fence_after();
-                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * P_BN + half_n * (P_BN / 2);
+                const uint32_t d_tmem = tmem_base + acc * P_BN;
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % P_STAGES;
+                    const uint32_t ph = (it / P_STAGES) & 1;
+                    mbar_wait(&bars[PB_FULL + s], ph, wctx, PB_FULL + s);
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * P_STAGE_BYTES);
+                    const uint32_t b_addr = a_addr + P_A_BYTES;
 #pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld32(t_row + ch * 64, r0);
-                    tmem_ld32(t_row + ch * 64 + 32, r1);
-                    tc_wait_ld();
-                    if (ch == 1) {
-                        // both chunks of this accumulator half are in registers: hand the accumulator back to the leader's MMA warp
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-                            if (leader) mbar_arrive(&bars[PB_TEMPTY + acc]);
-                            else remote_arrive_cta(map_to_rank(smem_u32(&bars[PB_TEMPTY + acc]), 0));
-                        }
+                    for (int kk = 0; kk < P_BK / 16; ++kk) {
+                        const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
+                        const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, P_BK * 64 * 2, 1024);
+                        mma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                     }
-                    const int col0 = colbase + ch * 64;
-                    if (col0 < n && row0 < m) {
-                        if (lane == 0) tma_store_wait_read();
-                        __syncwarp();
+                    // the stage is free in both blocks: one commit per block's barrier
+                    tc_commit_pair(smem_u32(&bars[PB_EMPTY + s]));
+                    tc_commit_pair(map_to_rank(smem_u32(&bars[PB_EMPTY + s]), 1));
+                }
+                tc_commit_pair(smem_u32(&bars[PB_TFULL + acc]));
+                tc_commit_pair(map_to_rank(smem_u32(&bars[PB_TFULL + acc]), 1));
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue (both blocks)
+        const int quarter = warp & 3, half_n = warp >> 2;
+        unsigned char* slab = slabs + warp * P_SLAB_BYTES;
+        const bool mute = failure_reported(status);
+        int local = 0;
+        for (int t = pair; t < num_tiles; t += pairs, ++local) {
+            const int acc = local & 1;
+            const uint32_t acc_ph = (local >> 1) & 1;
+            const int m0 = (t / tiles_n) * (2 * P_BM) + static_cast<int>(rank) * P_BM, n0 = (t % tiles_n) * P_BN;
+            const int row0 = m0 + quarter * 32;
+            const int row = row0 + lane;
+            const int colbase = n0 + half_n * (P_BN / 2);
+            uint4 res[2][8];
+            if (EPI == STOF_EPI_BIAS_RESIDUAL) {
 #pragma unroll
-                        for (int g = 0; g < 8; ++g) {
-                            const uint32_t* src = (g < 4) ? &r0[8 * g] : &r1[8 * (g - 4)];
-                            const int col = col0 + 8 * g;
-                            float2 v[4];
+                for (int ch = 0; ch < 2; ++ch)
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(src[2 * j]), __uint_as_float(src[2 * j + 1]));
-                            if (bias != nullptr && col < n) {
-                                const uint4 bu = __ldg(reinterpret_cast<const uint4*>(bias + col));
-                                const __half2* bh = reinterpret_cast<const __half2*>(&bu);
+                    for (int g = 0; g < 8; ++g) {
+                        const int col = colbase + ch * 64 + g * 8;
+                        res[ch][g] = (row < m && col < n) ? __ldg(reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * ldr + col))
+                                                          : make_uint4(0u, 0u, 0u, 0u);
+                    }
+            }
+            mbar_wait(&bars[PB_TFULL + acc], acc_ph, wctx, PB_TFULL + acc);
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * P_BN + half_n * (P_BN / 2);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float2 f = __half22float2(bh[j]);
-                                    v[j] = add2(v[j], pk2(f.x, f.y));
-                                }
+            for (int ch = 0; ch < 2; ++ch) {
+                uint32_t r0[32], r1[32];
+                tmem_ld32(t_row + ch * 64, r0);
+                tmem_ld32(t_row + ch * 64 + 32, r1);
+                tc_wait_ld();
+                if (ch == 1) {
+                    // both chunks of this accumulator half are in registers: hand the accumulator back to the leader's MMA warp
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (leader) mbar_arrive(&bars[PB_TEMPTY + acc]);
+                        else remote_arrive_cta(map_to_rank(smem_u32(&bars[PB_TEMPTY + acc]), 0));
+                    }
+                }
+                const int col0 = colbase + ch * 64;
+                if (col0 < n && row0 < m) {
+                    if (lane == 0) tma_store_wait_read();
+                    __syncwarp();
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const uint32_t* src = (g < 4) ? &r0[8 * g] : &r1[8 * (g - 4)];
+                        const int col = col0 + 8 * g;
+                        float2 v[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(src[2 * j]), __uint_as_float(src[2 * j + 1]));
+                        if (bias != nullptr && col < n) {
+                            const uint4 bu = __ldg(reinterpret_cast<const uint4*>(bias + col));
+                            const __half2* bh = reinterpret_cast<const __half2*>(&bu);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __half22float2(bh[j]);
+                                v[j] = add2(v[j], pk2(f.x, f.y));
                             }
-                            if (EPI == STOF_EPI_BIAS_GELU_ERF) {
+                        }
+                        if (EPI == STOF_EPI_BIAS_GELU_ERF) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) v[j] = gelu_erf2(v[j]);
-                            } else if (EPI == STOF_EPI_BIAS_GELU_TANH) {
+                            for (int j = 0; j < 4; ++j) v[j] = gelu_erf2(v[j]);
+                        } else if (EPI == STOF_EPI_BIAS_GELU_TANH) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) v[j] = gelu_tanh2(v[j]);
-                            } else if (EPI == STOF_EPI_BIAS_RELU) {
+                            for (int j = 0; j < 4; ++j) v[j] = gelu_tanh2(v[j]);
+                        } else if (EPI == STOF_EPI_BIAS_RELU) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    float x0, x1;
-                                    upk2(v[j], x0, x1);
-                                    v[j] = pk2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
-                                }
-                            } else if (EPI == STOF_EPI_BIAS_RESIDUAL) {
-                                const __half2* rh = reinterpret_cast<const __half2*>(&res[ch][g]);
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float2 f = __half22float2(rh[j]);
-                                    v[j] = add2(v[j], pk2(f.x, f.y));
-                                }
+                            for (int j = 0; j < 4; ++j) {
+                                float x0, x1;
+                                upk2(v[j], x0, x1);
+                                v[j] = pk2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
                             }
-                            uint4 o;
-                            float lo, hi;
-                            upk2(v[0], lo, hi); o.x = pack_half2(lo, hi);
-                            upk2(v[1], lo, hi); o.y = pack_half2(lo, hi);
-                            upk2(v[2], lo, hi); o.z = pack_half2(lo, hi);
-                            upk2(v[3], lo, hi); o.w = pack_half2(lo, hi);
-                            *reinterpret_cast<uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4)) = o;
+                        } else if (EPI == STOF_EPI_BIAS_RESIDUAL) {
+                            const __half2* rh = reinterpret_cast<const __half2*>(&res[ch][g]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __half22float2(rh[j]);
+                                v[j] = add2(v[j], pk2(f.x, f.y));
+                            }
                         }
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_2d(&map_c, slab, col0, row0);
-                            tma_store_commit();
-                        }
+                        uint4 o;
+                        float lo, hi;
+                        upk2(v[0], lo, hi); o.x = pack_half2(lo, hi);
+                        upk2(v[1], lo, hi); o.y = pack_half2(lo, hi);
+                        upk2(v[2], lo, hi); o.z = pack_half2(lo, hi);
+                        upk2(v[3], lo, hi); o.w = pack_half2(lo, hi);
+                        *reinterpret_cast<uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4)) = o;
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && !mute) {
+                        tma_store_2d(&map_c, slab, col0, row0);
+                        tma_store_commit();
                     }
                 }
             }
-            if (lane == 0) tma_store_wait_all();
         }
+        if (lane == 0) tma_store_wait_all();
     }
     // neither block leaves while its peer may still signal one of its barriers, read its shared memory or write its tensor memory
     tc_fence_before();

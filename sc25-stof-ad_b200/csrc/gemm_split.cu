@@ -97,7 +97,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     } else if (warp == EPI_WARPS) {
         if (elect_one()) split_prefetch<BN>(map_a, map_w, n0, kb0, kb1, stages);
     } else if (threadIdx.x == 0) {
-        *abort_flag = (status != nullptr && *status != 0) ? 1 : 0;
+        *abort_flag = 0;
         for (int i = 0; i < stages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -117,95 +117,91 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const bool run = *abort_flag == 0;           // as the kernel started: every warp takes the same way through the barriers below
-    if (run) {
-        if (warp == EPI_WARPS) {
-            split_produce<Shape, BN>(map_a, map_w, smem, full, empty, m0, n0, kb0, kb1, stages, wctx);
-        } else if (warp == EPI_WARPS + 1) {
-            split_multiply<Shape, BM, BN>(smem, full, empty, tfull, tmem_base, kb0, kb1, stages, wctx);
-        } else {
-            grid_dependency_wait();
-            const int rows = BM / split, row_lo = rank * rows;        // the rows this block finishes
-            stage_vector(s_bias, bias != nullptr ? bias + n0 : nullptr, n - n0, BN, 0u, 0);
-            if (RES) stage_residual<Shape>(s_res, residual, ldr, m0, n0, m, n, row_lo, rows);
-            copy_async_wait();
-            epilogue_barrier<Shape::EPI_THREADS>();
-            const int quarter = warp & 3, part = warp >> 2;
-            const bool mine = BM == 128 || lane < 16;
-            const int lrow = BM == 128 ? quarter * 32 + lane : quarter * 16 + (lane & 15);
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
-            mbar_wait_addr(smem_u32(tfull), 0, wctx, 2 * stages);
-            tc_fence_after();
-            if (split == 1) {
-                const int row = m0 + lrow;
-                const bool live = mine && row < m;
-                __half* out = c + static_cast<size_t>(row) * ldc + n0;
-#pragma unroll 1
-                for (int g0 = part * 8; g0 < part * 8 + 8; g0 += 2) {
-                    uint32_t r[16];
-                    tmem_ld16(t_row + (g0 & 7) * 8, r);
-                    tc_wait_ld();
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int g = g0 + h;
-                        float2 v[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(r[8 * h + 2 * j]), __uint_as_float(r[8 * h + 2 * j + 1]));
-                        uint4 res = make_uint4(0u, 0u, 0u, 0u);
-                        if (RES) res = *reinterpret_cast<const uint4*>(s_res + Shape::residual_at(lrow, g));
-                        const uint4 o = finish8<EPI>(v, reinterpret_cast<const uint4*>(s_bias)[g], res);
-                        if (live && n0 + 8 * g < n) *reinterpret_cast<uint4*>(out + 8 * g) = o;
-                    }
-                }
-            } else {
-                // a row of the partial tile, 16 bytes at a time; the pitch keeps eight lanes on different banks
-                float* own = reinterpret_cast<float*>(smem);
-                float* prow = own + lrow * Smem::PITCH + part * 64;
-#pragma unroll 1
-                for (int c0 = 0; c0 < 64; c0 += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(t_row + c0, r);
-                    tc_wait_ld();
-                    if (mine)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(prow + c0 + 4 * i) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-                }
-                const float* parts = reinterpret_cast<const float*>(smem + Smem::received_at(stages));
-                const int part_floats = Smem::part_bytes(split) / 4;
-                fence_proxy_async_smem();
-                epilogue_barrier<Shape::EPI_THREADS>();                  // the partial tile is written
-                if (static_cast<int>(threadIdx.x) < split && static_cast<int>(threadIdx.x) != rank) {
-                    // this block's part comes at place `rank`, or rank - 1 behind the receiver's own
-                    const int to = static_cast<int>(threadIdx.x), place = rank < to ? rank : rank - 1;
-                    bulk_copy_to_peer(map_to_rank(smem_u32(parts + place * part_floats), static_cast<uint32_t>(to)), smem_u32(own + to * part_floats),
-                                      static_cast<uint32_t>(Smem::part_bytes(split)), map_to_rank(smem_u32(received), static_cast<uint32_t>(to)));
-                }
-                __syncwarp();
-                mbar_wait_addr(smem_u32(received), 0, wctx, 2 * stages + 1);
-                // output pieces of 8 columns, eight or sixteen neighbouring threads to a row
-#pragma unroll 1
-                for (int i = threadIdx.x; i < rows * Shape::CHUNKS; i += Shape::EPI_THREADS) {
-                    const int lr = i / Shape::CHUNKS, g = i % Shape::CHUNKS, row = m0 + row_lo + lr;
-                    const int at = lr * Smem::PITCH + 8 * g;
-                    float2 v[4] = {};
-#pragma unroll 1
-                    for (int p = 0; p < split; ++p) {
-                        const float* from = (p == rank ? own + rank * part_floats : parts + (p < rank ? p : p - 1) * part_floats) + at;
-                        const float4 x = *reinterpret_cast<const float4*>(from), y = *reinterpret_cast<const float4*>(from + 4);
-                        v[0] = add2(v[0], pk2(x.x, x.y));
-                        v[1] = add2(v[1], pk2(x.z, x.w));
-                        v[2] = add2(v[2], pk2(y.x, y.y));
-                        v[3] = add2(v[3], pk2(y.z, y.w));
-                    }
-                    uint4 res = make_uint4(0u, 0u, 0u, 0u);
-                    if (RES) res = *reinterpret_cast<const uint4*>(s_res + Shape::residual_at(row_lo + lr, g));
-                    const uint4 o = finish8<EPI>(v, reinterpret_cast<const uint4*>(s_bias)[g], res);
-                    if (row < m && n0 + 8 * g < n) *reinterpret_cast<uint4*>(c + static_cast<size_t>(row) * ldc + n0 + 8 * g) = o;
-                }
-            }
-        }
+    if (warp == EPI_WARPS) {
+        split_produce<Shape, BN>(map_a, map_w, smem, full, empty, m0, n0, kb0, kb1, stages, wctx);
+    } else if (warp == EPI_WARPS + 1) {
+        split_multiply<Shape, BM, BN>(smem, full, empty, tfull, tmem_base, kb0, kb1, stages, wctx);
     } else {
         grid_dependency_wait();
+        const bool mute = failure_reported(status);
+        const int rows = BM / split, row_lo = rank * rows;        // the rows this block finishes
+        stage_vector(s_bias, bias != nullptr ? bias + n0 : nullptr, n - n0, BN, 0u, 0);
+        if (RES) stage_residual<Shape>(s_res, residual, ldr, m0, n0, m, n, row_lo, rows);
+        copy_async_wait();
+        epilogue_barrier<Shape::EPI_THREADS>();
+        const int quarter = warp & 3, part = warp >> 2;
+        const bool mine = BM == 128 || lane < 16;
+        const int lrow = BM == 128 ? quarter * 32 + lane : quarter * 16 + (lane & 15);
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
+        mbar_wait_addr(smem_u32(tfull), 0, wctx, 2 * stages);
+        tc_fence_after();
+        if (split == 1) {
+            const int row = m0 + lrow;
+            const bool live = mine && row < m && !mute;
+            __half* out = c + static_cast<size_t>(row) * ldc + n0;
+#pragma unroll 1
+            for (int g0 = part * 8; g0 < part * 8 + 8; g0 += 2) {
+                uint32_t r[16];
+                tmem_ld16(t_row + (g0 & 7) * 8, r);
+                tc_wait_ld();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int g = g0 + h;
+                    float2 v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(r[8 * h + 2 * j]), __uint_as_float(r[8 * h + 2 * j + 1]));
+                    uint4 res = make_uint4(0u, 0u, 0u, 0u);
+                    if (RES) res = *reinterpret_cast<const uint4*>(s_res + Shape::residual_at(lrow, g));
+                    const uint4 o = finish8<EPI>(v, reinterpret_cast<const uint4*>(s_bias)[g], res);
+                    if (live && n0 + 8 * g < n) *reinterpret_cast<uint4*>(out + 8 * g) = o;
+                }
+            }
+        } else {
+            // a row of the partial tile, 16 bytes at a time; the pitch keeps eight lanes on different banks
+            float* own = reinterpret_cast<float*>(smem);
+            float* prow = own + lrow * Smem::PITCH + part * 64;
+#pragma unroll 1
+            for (int c0 = 0; c0 < 64; c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(t_row + c0, r);
+                tc_wait_ld();
+                if (mine)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(prow + c0 + 4 * i) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+            }
+            const float* parts = reinterpret_cast<const float*>(smem + Smem::received_at(stages));
+            const int part_floats = Smem::part_bytes(split) / 4;
+            fence_proxy_async_smem();
+            epilogue_barrier<Shape::EPI_THREADS>();                  // the partial tile is written
+            if (static_cast<int>(threadIdx.x) < split && static_cast<int>(threadIdx.x) != rank) {
+                // this block's part comes at place `rank`, or rank - 1 behind the receiver's own
+                const int to = static_cast<int>(threadIdx.x), place = rank < to ? rank : rank - 1;
+                bulk_copy_to_peer(map_to_rank(smem_u32(parts + place * part_floats), static_cast<uint32_t>(to)), smem_u32(own + to * part_floats),
+                                  static_cast<uint32_t>(Smem::part_bytes(split)), map_to_rank(smem_u32(received), static_cast<uint32_t>(to)));
+            }
+            __syncwarp();
+            mbar_wait_addr(smem_u32(received), 0, wctx, 2 * stages + 1);
+            // output pieces of 8 columns, eight or sixteen neighbouring threads to a row
+#pragma unroll 1
+            for (int i = threadIdx.x; i < rows * Shape::CHUNKS; i += Shape::EPI_THREADS) {
+                const int lr = i / Shape::CHUNKS, g = i % Shape::CHUNKS, row = m0 + row_lo + lr;
+                const int at = lr * Smem::PITCH + 8 * g;
+                float2 v[4] = {};
+#pragma unroll 1
+                for (int p = 0; p < split; ++p) {
+                    const float* from = (p == rank ? own + rank * part_floats : parts + (p < rank ? p : p - 1) * part_floats) + at;
+                    const float4 x = *reinterpret_cast<const float4*>(from), y = *reinterpret_cast<const float4*>(from + 4);
+                    v[0] = add2(v[0], pk2(x.x, x.y));
+                    v[1] = add2(v[1], pk2(x.z, x.w));
+                    v[2] = add2(v[2], pk2(y.x, y.y));
+                    v[3] = add2(v[3], pk2(y.z, y.w));
+                }
+                uint4 res = make_uint4(0u, 0u, 0u, 0u);
+                if (RES) res = *reinterpret_cast<const uint4*>(s_res + Shape::residual_at(row_lo + lr, g));
+                const uint4 o = finish8<EPI>(v, reinterpret_cast<const uint4*>(s_bias)[g], res);
+                if (row < m && n0 + 8 * g < n && !mute) *reinterpret_cast<uint4*>(c + static_cast<size_t>(row) * ldc + n0 + 8 * g) = o;
+            }
+        }
     }
     tc_fence_before();
     // A block has waited for all that its peers send it, but a peer may still be reading out what this one sends from here

@@ -56,7 +56,7 @@ gemm_split_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == EPI_WARPS) {
         if (elect_one()) split_prefetch<BN>(map_a, map_w, n0, 0, kblocks, stages);
     } else if (threadIdx.x == 0) {
-        *abort_flag = (status != nullptr && *status != 0) ? 1 : 0;
+        *abort_flag = 0;
         for (int i = 0; i < stages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -71,19 +71,13 @@ gemm_split_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     cluster_sync_all();                          // every block's barriers exist before a peer's copy reports to them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // The status word is read by every block on its own.  A block that sat out would leave its peers waiting for its statistics,
-    // so all of them run, and a block that found the word set writes nothing.
-    const bool mute = *abort_flag != 0;
-    __syncthreads();
-    if (threadIdx.x == 0) *abort_flag = 0;
-    __syncthreads();
-
     if (warp == EPI_WARPS) {
         split_produce<Shape, BN>(map_a, map_w, smem, full, empty, m0, n0, 0, kblocks, stages, wctx);
     } else if (warp == EPI_WARPS + 1) {
         split_multiply<Shape, BM, BN>(smem, full, empty, tfull, tmem_base, 0, kblocks, stages, wctx);
     } else {
         grid_dependency_wait();
+        const bool mute = failure_reported(status);
         const uint4* s_bias = reinterpret_cast<const uint4*>(s_vec);
         stage_vector(s_vec, bias != nullptr ? bias + n0 : nullptr, BN, BN, 0u, 0);
         stage_vector(s_vec + 2 * BN, gamma != nullptr ? gamma + n0 : nullptr, BN, BN, 0x3C003C00u, 32);       // 1.0

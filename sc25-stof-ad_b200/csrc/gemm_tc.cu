@@ -50,7 +50,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const WaitCtx wctx{abort_flag, status};
 
     if (threadIdx.x == 0) {
-        *abort_flag = (status != nullptr && *status != 0) ? 1 : 0;
+        *abort_flag = 0;
         for (int i = 0; i < G_STAGES; ++i) {
             mbar_init(&bars[BAR_FULL + i], 1);
             mbar_init(&bars[BAR_EMPTY + i], 1);
@@ -72,157 +72,156 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     grid_dependency_wait();
     grid_launch_dependents();
 
-    if (*abort_flag == 0) {
-        if (warp == G_EPI_WARPS) {
-            // ------------------------------------------------------------------ TMA producer
-            if (elect_one()) {
-                tma_prefetch_desc(&map_a);
-                tma_prefetch_desc(&map_w);
-                int it = 0;
-                for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-                    const int m0 = (t / tiles_n) * G_BM, n0 = (t % tiles_n) * G_BN;
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % G_STAGES;
-                        const uint32_t ph = (it / G_STAGES) & 1;
-                        mbar_wait(&bars[BAR_EMPTY + s], ph ^ 1, wctx, BAR_EMPTY + s);
-                        unsigned char* a_dst = smem + s * G_STAGE_BYTES;
-                        unsigned char* b_dst = a_dst + G_A_BYTES;
-                        mbar_arrive_expect_tx(&bars[BAR_FULL + s], G_STAGE_BYTES);
-                        tma_load_2d(a_dst, &map_a, &bars[BAR_FULL + s], kb * G_BK, m0);
+    if (warp == G_EPI_WARPS) {
+        // ------------------------------------------------------------------ TMA producer
+        if (elect_one()) {
+            tma_prefetch_desc(&map_a);
+            tma_prefetch_desc(&map_w);
+            int it = 0;
+            for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+                const int m0 = (t / tiles_n) * G_BM, n0 = (t % tiles_n) * G_BN;
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % G_STAGES;
+                    const uint32_t ph = (it / G_STAGES) & 1;
+                    mbar_wait(&bars[BAR_EMPTY + s], ph ^ 1, wctx, BAR_EMPTY + s);
+                    unsigned char* a_dst = smem + s * G_STAGE_BYTES;
+                    unsigned char* b_dst = a_dst + G_A_BYTES;
+                    mbar_arrive_expect_tx(&bars[BAR_FULL + s], G_STAGE_BYTES);
+                    tma_load_2d(a_dst, &map_a, &bars[BAR_FULL + s], kb * G_BK, m0);
 #pragma unroll
-                        for (int j = 0; j < G_BN / 64; ++j)
-                            tma_load_2d(b_dst + j * (G_BK * 64 * 2), &map_w, &bars[BAR_FULL + s], n0 + 64 * j, kb * G_BK);
-                    }
+                    for (int j = 0; j < G_BN / 64; ++j)
+                        tma_load_2d(b_dst + j * (G_BK * 64 * 2), &map_w, &bars[BAR_FULL + s], n0 + 64 * j, kb * G_BK);
                 }
             }
-        } else if (warp == G_EPI_WARPS + 1) {
-            // ------------------------------------------------------------------ MMA issuer
-            if (elect_one()) {
-                constexpr uint32_t idesc = make_idesc_f16(G_BM, G_BN, /*b_mn_major=*/true);
-                int it = 0, local = 0;
-                for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++local) {
-                    const int acc = local & 1;
-                    const uint32_t acc_ph = (local >> 1) & 1;
-                    mbar_wait(&bars[BAR_TEMPTY + acc], acc_ph ^ 1, wctx, BAR_TEMPTY + acc);
-                    tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * G_BN;
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % G_STAGES;
-                        const uint32_t ph = (it / G_STAGES) & 1;
-                        mbar_wait(&bars[BAR_FULL + s], ph, wctx, BAR_FULL + s);
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_u32(smem + s * G_STAGE_BYTES);
-                        const uint32_t b_addr = a_addr + G_A_BYTES;
-#pragma unroll
-                        for (int kk = 0; kk < G_BK / 16; ++kk) {
-                            const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-                            const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, G_BK * 64 * 2, 1024);
-                            mma_f16_ss(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-                        }
-                        tc_commit(&bars[BAR_EMPTY + s]);
-                    }
-                    tc_commit(&bars[BAR_TFULL + acc]);
-                }
-            }
-        } else {
-            // ------------------------------------------------------------------ epilogue
-            const int quarter = warp & 3, half_n = warp >> 2;
-            unsigned char* slab = slabs + warp * G_SLAB_BYTES;
-            int local = 0;
+        }
+    } else if (warp == G_EPI_WARPS + 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        if (elect_one()) {
+            constexpr uint32_t idesc = make_idesc_f16(G_BM, G_BN, /*b_mn_major=*/true);
+            int it = 0, local = 0;
             for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++local) {
                 const int acc = local & 1;
                 const uint32_t acc_ph = (local >> 1) & 1;
-                const int m0 = (t / tiles_n) * G_BM, n0 = (t % tiles_n) * G_BN;
-                const int row0 = m0 + quarter * 32;
-                const int row = row0 + lane;
-                const int colbase = n0 + half_n * (G_BN / 2);
-                // the residual does not depend on the accumulator: its loads are in flight while the tile's MMAs finish
-                uint4 res[2][8];
-                if (EPI == STOF_EPI_BIAS_RESIDUAL) {
-#pragma unroll
-                    for (int ch = 0; ch < 2; ++ch)
-#pragma unroll
-                        for (int g = 0; g < 8; ++g) {
-                            const int col = colbase + ch * 64 + g * 8;
-                            res[ch][g] = (row < m && col < n) ? __ldg(reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * ldr + col))
-                                                              : make_uint4(0u, 0u, 0u, 0u);
-                        }
-                }
-                mbar_wait(&bars[BAR_TFULL + acc], acc_ph, wctx, BAR_TFULL + acc);
+                mbar_wait(&bars[BAR_TEMPTY + acc], acc_ph ^ 1, wctx, BAR_TEMPTY + acc);
                 tc_fence_after();
-                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * G_BN + half_n * (G_BN / 2);
+                const uint32_t d_tmem = tmem_base + acc * G_BN;
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const int s = it % G_STAGES;
+                    const uint32_t ph = (it / G_STAGES) & 1;
+                    mbar_wait(&bars[BAR_FULL + s], ph, wctx, BAR_FULL + s);
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * G_STAGE_BYTES);
+                    const uint32_t b_addr = a_addr + G_A_BYTES;
 #pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld32(t_row + ch * 64, r0);
-                    tmem_ld32(t_row + ch * 64 + 32, r1);
-                    tc_wait_ld();
-                    if (ch == 1) {
-                        // both chunks of this accumulator half are in registers: hand the accumulator back to the MMA warp
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bars[BAR_TEMPTY + acc]);
+                    for (int kk = 0; kk < G_BK / 16; ++kk) {
+                        const uint64_t a_desc = make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
+                        const uint64_t b_desc = make_smem_desc_sw128(b_addr + kk * 2048, G_BK * 64 * 2, 1024);
+                        mma_f16_ss(d_tmem, a_desc, b_desc, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                     }
-                    const int col0 = colbase + ch * 64;
-                    if (col0 < n && row0 < m) {
-                        if (lane == 0) tma_store_wait_read();             // the slab's previous store has been read out
-                        __syncwarp();
+                    tc_commit(&bars[BAR_EMPTY + s]);
+                }
+                tc_commit(&bars[BAR_TFULL + acc]);
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue
+        const int quarter = warp & 3, half_n = warp >> 2;
+        unsigned char* slab = slabs + warp * G_SLAB_BYTES;
+        const bool mute = failure_reported(status);
+        int local = 0;
+        for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++local) {
+            const int acc = local & 1;
+            const uint32_t acc_ph = (local >> 1) & 1;
+            const int m0 = (t / tiles_n) * G_BM, n0 = (t % tiles_n) * G_BN;
+            const int row0 = m0 + quarter * 32;
+            const int row = row0 + lane;
+            const int colbase = n0 + half_n * (G_BN / 2);
+            // the residual does not depend on the accumulator: its loads are in flight while the tile's MMAs finish
+            uint4 res[2][8];
+            if (EPI == STOF_EPI_BIAS_RESIDUAL) {
 #pragma unroll
-                        for (int g = 0; g < 8; ++g) {                     // 8 columns = one 16-byte chunk of the output row
-                            const uint32_t* src = (g < 4) ? &r0[8 * g] : &r1[8 * (g - 4)];
-                            const int col = col0 + 8 * g;
-                            float2 v[4];
+                for (int ch = 0; ch < 2; ++ch)
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(src[2 * j]), __uint_as_float(src[2 * j + 1]));
-                            if (bias != nullptr && col < n) {
-                                const uint4 bu = __ldg(reinterpret_cast<const uint4*>(bias + col));
-                                const __half2* bh = reinterpret_cast<const __half2*>(&bu);
+                    for (int g = 0; g < 8; ++g) {
+                        const int col = colbase + ch * 64 + g * 8;
+                        res[ch][g] = (row < m && col < n) ? __ldg(reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * ldr + col))
+                                                          : make_uint4(0u, 0u, 0u, 0u);
+                    }
+            }
+            mbar_wait(&bars[BAR_TFULL + acc], acc_ph, wctx, BAR_TFULL + acc);
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * G_BN + half_n * (G_BN / 2);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float2 f = __half22float2(bh[j]);
-                                    v[j] = add2(v[j], pk2(f.x, f.y));
-                                }
+            for (int ch = 0; ch < 2; ++ch) {
+                uint32_t r0[32], r1[32];
+                tmem_ld32(t_row + ch * 64, r0);
+                tmem_ld32(t_row + ch * 64 + 32, r1);
+                tc_wait_ld();
+                if (ch == 1) {
+                    // both chunks of this accumulator half are in registers: hand the accumulator back to the MMA warp
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[BAR_TEMPTY + acc]);
+                }
+                const int col0 = colbase + ch * 64;
+                if (col0 < n && row0 < m) {
+                    if (lane == 0) tma_store_wait_read();             // the slab's previous store has been read out
+                    __syncwarp();
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {                     // 8 columns = one 16-byte chunk of the output row
+                        const uint32_t* src = (g < 4) ? &r0[8 * g] : &r1[8 * (g - 4)];
+                        const int col = col0 + 8 * g;
+                        float2 v[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] = pk2(__uint_as_float(src[2 * j]), __uint_as_float(src[2 * j + 1]));
+                        if (bias != nullptr && col < n) {
+                            const uint4 bu = __ldg(reinterpret_cast<const uint4*>(bias + col));
+                            const __half2* bh = reinterpret_cast<const __half2*>(&bu);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __half22float2(bh[j]);
+                                v[j] = add2(v[j], pk2(f.x, f.y));
                             }
-                            if (EPI == STOF_EPI_BIAS_GELU_ERF) {
+                        }
+                        if (EPI == STOF_EPI_BIAS_GELU_ERF) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) v[j] = gelu_erf2(v[j]);
-                            } else if (EPI == STOF_EPI_BIAS_GELU_TANH) {
+                            for (int j = 0; j < 4; ++j) v[j] = gelu_erf2(v[j]);
+                        } else if (EPI == STOF_EPI_BIAS_GELU_TANH) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) v[j] = gelu_tanh2(v[j]);
-                            } else if (EPI == STOF_EPI_BIAS_RELU) {
+                            for (int j = 0; j < 4; ++j) v[j] = gelu_tanh2(v[j]);
+                        } else if (EPI == STOF_EPI_BIAS_RELU) {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    float x0, x1;
-                                    upk2(v[j], x0, x1);
-                                    v[j] = pk2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
-                                }
-                            } else if (EPI == STOF_EPI_BIAS_RESIDUAL) {
-                                const __half2* rh = reinterpret_cast<const __half2*>(&res[ch][g]);
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float2 f = __half22float2(rh[j]);
-                                    v[j] = add2(v[j], pk2(f.x, f.y));
-                                }
+                            for (int j = 0; j < 4; ++j) {
+                                float x0, x1;
+                                upk2(v[j], x0, x1);
+                                v[j] = pk2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
                             }
-                            uint4 o;
-                            float lo, hi;
-                            upk2(v[0], lo, hi); o.x = pack_half2(lo, hi);
-                            upk2(v[1], lo, hi); o.y = pack_half2(lo, hi);
-                            upk2(v[2], lo, hi); o.z = pack_half2(lo, hi);
-                            upk2(v[3], lo, hi); o.w = pack_half2(lo, hi);
-                            *reinterpret_cast<uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4)) = o;
+                        } else if (EPI == STOF_EPI_BIAS_RESIDUAL) {
+                            const __half2* rh = reinterpret_cast<const __half2*>(&res[ch][g]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __half22float2(rh[j]);
+                                v[j] = add2(v[j], pk2(f.x, f.y));
+                            }
                         }
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_2d(&map_c, slab, col0, row0);       // rows / columns beyond the matrix are clipped by the tensor map
-                            tma_store_commit();
-                        }
+                        uint4 o;
+                        float lo, hi;
+                        upk2(v[0], lo, hi); o.x = pack_half2(lo, hi);
+                        upk2(v[1], lo, hi); o.y = pack_half2(lo, hi);
+                        upk2(v[2], lo, hi); o.z = pack_half2(lo, hi);
+                        upk2(v[3], lo, hi); o.w = pack_half2(lo, hi);
+                        *reinterpret_cast<uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4)) = o;
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && !mute) {
+                        tma_store_2d(&map_c, slab, col0, row0);       // rows / columns beyond the matrix are clipped by the tensor map
+                        tma_store_commit();
                     }
                 }
             }
-            if (lane == 0) tma_store_wait_all();
         }
+        if (lane == 0) tma_store_wait_all();
     }
     tc_fence_before();
     __syncthreads();

@@ -41,6 +41,11 @@ __device__ __forceinline__ bool elect_one() {
 // visible, and only then reads or writes global memory that a kernel may touch.  EVERY thread block has to come through
 // grid_dependency_wait before it exits: the next kernel's wait covers this one only, and through this one's wait the ones before.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Has a kernel reported a failure?  For threads that have come through grid_dependency_wait: before it the kernel that is about to
+// report may still run.  The GEMM kernels ask in their epilogue, under the first products, and write nothing where the answer is yes;
+// all else they do as ever.  (A thread block, or one of a cluster, that left at once would leave its peers waiting for it, as blocks
+// may see the word differently.)
+__device__ __forceinline__ bool failure_reported(const int* status) { return status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0; }
 // From here on the next kernel of the stream may be given whatever this one leaves free of the GPU.  Comes after the wait: what
 // lies two launches back or more is then complete before a kernel starts, and only the kernel just before it has to be waited for.
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

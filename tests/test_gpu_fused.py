@@ -404,3 +404,26 @@ def test_layernorm_epilogue_keeps_its_sums_in_fp32_at_every_row_count(m, n, k):
     got = stof_b200.gemm_bias_residual_layernorm(a.cuda(), w.cuda(), None, r.cuda(), None, None, 1e-12)
     want = of.gemm_bias_residual_layernorm(a, w, torch.zeros(n).half(), r, torch.ones(n).half(), torch.zeros(n).half(), 1e-12)
     assert _err(got, want) <= 4e-3
+
+
+@pytest.mark.parametrize("m,n,k,norm", [(64, 64, 64, False), (100, 768, 4096, False), (4096, 768, 72, False), (4096, 2560, 72, False), (65, 768, 136, True),
+                                        (8065, 1024, 72, True)])
+def test_gemms_write_nothing_once_a_failure_is_reported(m, n, k, norm):
+    """Small tiles, small tiles with K cut over a cluster, one-block and two-block kernel, both kernels with the LayerNorm: the output stays
+    as it was while the status word is set, with every block of a cluster taking part, and the word itself stays what it was."""
+    import stof_b200
+    from stof_b200 import _lib
+    a, w = _rand((m, k), 95).cuda(), _rand((k, n), 96, k ** -0.5).cuda()
+    call = (lambda out: stof_b200.gemm_bias_residual_layernorm(a, w, None, None, None, None, 1e-5, out=out)) if norm else \
+           (lambda out: stof_b200.gemm_bias(a, w, out=out))
+    want = call(None)
+    word = _lib.status_word(a.device)
+    out = torch.full_like(want, 7.0)
+    try:
+        word.fill_(0x0301)
+        call(out)
+        torch.cuda.synchronize()
+        assert (out == 7.0).all() and word.item() == 0x0301
+    finally:
+        word.zero_()
+    assert torch.equal(call(out), want)
