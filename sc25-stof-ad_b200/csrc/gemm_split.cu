@@ -123,10 +123,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         split_multiply<Shape, BM, BN>(smem, full, empty, tfull, tmem_base, kb0, kb1, stages, wctx);
     } else {
         grid_dependency_wait();
-        const bool mute = failure_reported(status);
         const int rows = BM / split, row_lo = rank * rows;        // the rows this block finishes
         stage_vector(s_bias, bias != nullptr ? bias + n0 : nullptr, n - n0, BN, 0u, 0);
         if (RES) stage_residual<Shape>(s_res, residual, ldr, m0, n0, m, n, row_lo, rows);
+        const bool mute = failure_reported(status);
         copy_async_wait();
         epilogue_barrier<Shape::EPI_THREADS>();
         const int quarter = warp & 3, part = warp >> 2;

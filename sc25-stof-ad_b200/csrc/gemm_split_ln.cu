@@ -77,12 +77,12 @@ gemm_split_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         split_multiply<Shape, BM, BN>(smem, full, empty, tfull, tmem_base, 0, kblocks, stages, wctx);
     } else {
         grid_dependency_wait();
-        const bool mute = failure_reported(status);
         const uint4* s_bias = reinterpret_cast<const uint4*>(s_vec);
         stage_vector(s_vec, bias != nullptr ? bias + n0 : nullptr, BN, BN, 0u, 0);
         stage_vector(s_vec + 2 * BN, gamma != nullptr ? gamma + n0 : nullptr, BN, BN, 0x3C003C00u, 32);       // 1.0
         stage_vector(s_vec + 4 * BN, beta != nullptr ? beta + n0 : nullptr, BN, BN, 0u, 64);
         stage_residual<Shape>(s_res, residual, ldr, m0, n0, m, cluster * BN, 0, BM);
+        const bool mute = failure_reported(status);
         copy_async_wait();
         epilogue_barrier<Shape::EPI_THREADS>();
         const int quarter = warp & 3, part = warp >> 2;
