@@ -306,7 +306,7 @@ struct ItemSource {
 __device__ __forceinline__ ItemSource item_source(const AttnParams& p) {
     ItemSource src;
     if (p.schedule != nullptr) {
-        const int b0 = __ldg(p.schedule + 1 + blockIdx.x), b1 = __ldg(p.schedule + 2 + blockIdx.x);
+        const int b0 = __ldca(p.schedule + 1 + blockIdx.x), b1 = __ldca(p.schedule + 2 + blockIdx.x);
         src.ids = p.schedule + 2 + gridDim.x + b0;
         src.count = b1 > b0 ? static_cast<unsigned>(b1 - b0) : 0u;
     } else {
@@ -319,7 +319,7 @@ __device__ __forceinline__ ItemSource item_source(const AttnParams& p) {
 constexpr unsigned A_NO_ITEM = 0xffffffffu;
 __device__ __forceinline__ unsigned fetch_item_id(unsigned k, const ItemSource& src) {
     if (k >= src.count) return A_NO_ITEM;
-    return src.ids != nullptr ? static_cast<unsigned>(__ldg(src.ids + k)) : blockIdx.x + k * gridDim.x;
+    return src.ids != nullptr ? static_cast<unsigned>(__ldca(src.ids + k)) : blockIdx.x + k * gridDim.x;
 }
 // Step two: the item's coordinates and its tile count.
 __device__ __forceinline__ Item decode_item(unsigned id, const AttnParams& p, const int2* sched) {
@@ -335,7 +335,7 @@ __device__ __forceinline__ Item decode_item(unsigned id, const AttnParams& p, co
         }
         const unsigned bh = id / static_cast<unsigned>(p.n_qtiles);
         it.qt = static_cast<int>(id - bh * static_cast<unsigned>(p.n_qtiles));
-        it.n = __ldg(reinterpret_cast<const int*>(p.plan + plan_off_nsteps()) + it.qt);
+        it.n = __ldca(reinterpret_cast<const int*>(p.plan + plan_off_nsteps()) + it.qt);
         it.batch = static_cast<int>(bh / p.heads);
         it.head = static_cast<int>(bh - it.batch * p.heads);
         return it;
@@ -347,7 +347,7 @@ __device__ __forceinline__ Item decode_item(unsigned id, const AttnParams& p, co
     const unsigned gsize = min(static_cast<unsigned>(A_GROUP_BH), p.bh_total - bh0);     // the tail group is smaller
     const unsigned rank = r / gsize;
     const unsigned bh = bh0 + (r - rank * gsize);
-    const int2 sc = __ldg(sched + rank);
+    const int2 sc = __ldca(sched + rank);
     it.qt = sc.x;
     it.n = sc.y;
     it.batch = static_cast<int>(bh / p.heads);
@@ -410,8 +410,8 @@ __device__ __noinline__ void mask_scores_in_tmem(uint32_t t_s, uint32_t cx, uint
         m[cg][1] = make_uint4(0u, 0u, 0u, 0u);
         if (code[cg] >= 2u) {
             const __half* mp = mask_row_ptr(part_block_mask, part_base, code[cg], bm_shift, bn, row_in_block, col0 + cg * 16);
-            m[cg][0] = __ldg(reinterpret_cast<const uint4*>(mp));
-            m[cg][1] = __ldg(reinterpret_cast<const uint4*>(mp + 8));
+            m[cg][0] = __ldca(reinterpret_cast<const uint4*>(mp));
+            m[cg][1] = __ldca(reinterpret_cast<const uint4*>(mp + 8));
         }
     }
 #pragma unroll
@@ -565,11 +565,11 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 auto settle = [&](Cursor& c) {
                     c.q.skip_empty(p, plan_sched);
                     c.item = c.q.cur;
-                    if (c.item.valid) c.word = __ldg(plan_steps + static_cast<size_t>(c.item.qt) * p.max_steps);
+                    if (c.item.valid) c.word = __ldca(plan_steps + static_cast<size_t>(c.item.qt) * p.max_steps);
                 };
                 auto advance = [&](Cursor& c) {
                     if (++c.j >= c.item.n) { c.j = 0; ++c.it; c.q.pop(p, plan_sched); settle(c); }
-                    else c.word = __ldg(plan_steps + static_cast<size_t>(c.item.qt) * p.max_steps + c.j);
+                    else c.word = __ldca(plan_steps + static_cast<size_t>(c.item.qt) * p.max_steps + c.j);
                 };
                 auto step_word = [&](const Cursor& c) { return c.word; };
                 Cursor kc, vc;
@@ -584,7 +584,7 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                         const int qb = kc.it % A_QBUFS;
                         mbar_wait(&bars[AB_Q_EMPTY + qb], static_cast<uint32_t>(((kc.it / A_QBUFS) & 1) ^ 1), wctx, AB_Q_EMPTY + qb);
                         // the item's two 64-row halves (the second may be missing; its rows then carry "absent" codes only)
-                        const int2 hr = __ldg(plan_halves + kc.item.qt);
+                        const int2 hr = __ldca(plan_halves + kc.item.qt);
                         unsigned char* qd = q_smem + qb * A_QBUF_BYTES;
                         uint64_t* qfull = &bars[AB_Q_FULL + qb];
                         mbar_arrive_expect_tx(qfull, hr.y >= 0 ? A_QBUF_BYTES : A_Q_BYTES / 2);
@@ -654,11 +654,11 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     c.valid = c.q.cur.valid;
                     c.n = c.q.cur.n;
                     c.qt = c.q.cur.qt;
-                    if (c.valid) c.word = __ldg(plan_steps + static_cast<size_t>(c.qt) * p.max_steps);
+                    if (c.valid) c.word = __ldca(plan_steps + static_cast<size_t>(c.qt) * p.max_steps);
                 };
                 auto advance = [&](Cursor& c) {
                     if (++c.j >= c.n) { c.j = 0; ++c.it; c.q.pop(p, plan_sched); settle(c); }
-                    else c.word = __ldg(plan_steps + static_cast<size_t>(c.qt) * p.max_steps + c.j);
+                    else c.word = __ldca(plan_steps + static_cast<size_t>(c.qt) * p.max_steps + c.j);
                 };
                 Cursor qk, pv;
                 qk.q.init(p, plan_sched);
@@ -747,11 +747,11 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             // per-item values that need global loads are fetched one item ahead (no dependent-load chain at item boundaries)
             // first sequence row of the 64-row half this thread works on (-1: the item has no such half)
             auto item_half = [&](const Item& x) -> int {
-                return x.valid ? __ldg(reinterpret_cast<const int*>(plan_halves) + 2 * x.qt + hsel) : -1;
+                return x.valid ? __ldca(reinterpret_cast<const int*>(plan_halves) + 2 * x.qt + hsel) : -1;
             };
             auto item_row_base = [&](const Item& x, int half_row) -> int {
                 const int r = half_row + rih;
-                return (x.valid && x.n > 0 && half_row >= 0 && r < p.seq_len) ? __ldg(p.part_row_ptr + (r >> p.bm_shift)) : 0;
+                return (x.valid && x.n > 0 && half_row >= 0 && r < p.seq_len) ? __ldca(p.part_row_ptr + (r >> p.bm_shift)) : 0;
             };
             auto item_codes = [&](const Item& x) -> const uint2* {
                 return reinterpret_cast<const uint2*>(plan_codes + (static_cast<size_t>(x.qt) * p.max_steps) * 32 + rg * 4);
@@ -782,7 +782,7 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             unsigned id_ahead = fetch_item_id(2, isrc);      // number of item k + 2, requested an item before it is decoded
             int half_row = item_half(cur_item), half1 = item_half(item1);
             int part_base = item_row_base(cur_item, half_row);
-            uint2 cw = (cur_item.valid && cur_item.n > 0) ? __ldg(item_codes(cur_item)) : make_uint2(0u, 0u);      // codes of step 0
+            uint2 cw = (cur_item.valid && cur_item.n > 0) ? __ldca(item_codes(cur_item)) : make_uint2(0u, 0u);      // codes of step 0
             for (unsigned k = 0; cur_item.valid; ++k) {
                 // the values of the items after this one; they replace the current ones at the end of the iteration
                 Item item2;
@@ -790,7 +790,7 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 uint2 cw1;
                 auto fetch_ahead = [&]() {
                     part_base1 = item_row_base(item1, half1);
-                    cw1 = (item1.valid && item1.n > 0) ? __ldg(item_codes(item1)) : make_uint2(0u, 0u);
+                    cw1 = (item1.valid && item1.n > 0) ? __ldca(item_codes(item1)) : make_uint2(0u, 0u);
                     item2 = decode_item(id_ahead, p, plan_sched);
                     id_ahead = fetch_item_id(k + 3, isrc);
                     half2 = item_half(item2);
@@ -817,7 +817,7 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                     const uint32_t bphase = sphase;
                     if (++sbuf == A_SBUF) { sbuf = 0; sphase ^= 1u; }
                     const uint2 cur = cw;
-                    if (j + 1 < n) cw = __ldg(my_codes + (j + 1) * 8);     // 32 codes = 64 B = 8 uint2 per step
+                    if (j + 1 < n) cw = __ldca(my_codes + (j + 1) * 8);     // 32 codes = 64 B = 8 uint2 per step
                     // class of this warp's 32 x 64 part of the step, put into the codes by the plan: the same value in every lane
                     const unsigned warp_class = cur.y >> 30;
                     const bool warp_absent = warp_class == 0u, warp_fast = warp_class == 1u;
@@ -835,7 +835,7 @@ block_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                         if (!warp_fast)
                             mask_scores_in_tmem(t_lane + A_COL_S + b * A_TKV, cur.x, cur.y, p.part_block_mask, part_base, p.bm_shift, p.bn,
                                                 (half_row + rih) & (p.bm - 1),
-                                                static_cast<int>((__ldg(plan_steps + static_cast<size_t>(cur_item.qt) * p.max_steps + j) >> (16 * hsel)) & 0xFFFFu) * A_TKV);
+                                                static_cast<int>((__ldca(plan_steps + static_cast<size_t>(cur_item.qt) * p.max_steps + j) >> (16 * hsel)) & 0xFFFFu) * A_TKV);
                         tmem_ld32(t_lane + A_COL_S + b * A_TKV, r0);
                         tmem_ld32(t_lane + A_COL_S + b * A_TKV + 32, r1);
                         tc_wait_ld();

@@ -67,8 +67,8 @@ __device__ __forceinline__ void store8(__half* p, const float (&f)[8]) {
 // 8192 rows of 768 9.5 -> 8.0 us.  Two blocks on an SM matter more than the last registers (hidden 768: 23 us with one of 152).
 template <int NCHUNK, int ROWS>
 __global__ void __launch_bounds__(LN_WARPS * 32, 2)
-layernorm_kernel(const __half* x, long long ldx, const __half* __restrict__ bias, const __half* __restrict__ residual,
-                 long long ldr, const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps, __half* y,
+layernorm_kernel(const __half* x, long long ldx, const __half* bias, const __half* residual,
+                 long long ldr, const __half* gamma, const __half* beta, float eps, __half* y,
                  long long ldy, int rows, int hidden, int* status) {
     extern __shared__ __align__(128) unsigned char ln_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -120,7 +120,7 @@ layernorm_kernel(const __half* x, long long ldx, const __half* __restrict__ bias
         constexpr int V = VECTORS_IN_REGS ? NCHUNK : 1;
         const uint4 zeros = make_uint4(0u, 0u, 0u, 0u), ones = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
         auto vec = [&](const __half* v, int i, const uint4& none) {
-            return v != nullptr ? __ldg(reinterpret_cast<const uint4*>(v + 8 * (lane + 32 * i))) : none;
+            return v != nullptr ? __ldca(reinterpret_cast<const uint4*>(v + 8 * (lane + 32 * i))) : none;
         };
         uint4 ub[V], ug[V], ut[V];
         if constexpr (VECTORS_IN_REGS) {

@@ -170,7 +170,7 @@ constexpr int CLASSIFY_FLIGHT = 8;            // independent 16-byte loads of a 
 
 template <bool F32>
 __global__ void __launch_bounds__(CLASSIFY_THREADS)
-classify_kernel(const void* __restrict__ mask, const Geometry geo, int* full_row_ptr, int* part_row_ptr, int* load_row_ptr, const Report report,
+classify_kernel(const void* mask, const Geometry geo, int* full_row_ptr, int* part_row_ptr, int* load_row_ptr, const Report report,
                 const Workspace ws, unsigned char* cls) {
     constexpr int EPC = F32 ? 4 : 8;                       // elements per 16-byte chunk
     constexpr unsigned ONE = F32 ? 0x3F800000u : 0x3C003C00u, MAG = F32 ? 0x7FFFFFFFu : 0x7FFF7FFFu;
@@ -204,7 +204,7 @@ classify_kernel(const void* __restrict__ mask, const Geometry geo, int* full_row
                 uint4 v[CLASSIFY_FLIGHT];
 #pragma unroll
                 for (int u = 0; u < CLASSIFY_FLIGHT; ++u)
-                    if (r + u * rows_at_once < bm) v[u] = __ldg(p + u * step);
+                    if (r + u * rows_at_once < bm) v[u] = __ldca(p + u * step);
 #pragma unroll
                 for (int u = 0; u < CLASSIFY_FLIGHT; ++u)
                     if (r + u * rows_at_once < bm) {
@@ -267,12 +267,12 @@ __device__ __forceinline__ uint4 mask_addend8(const void* mask, size_t src) {
     const __half one = __float2half(1.0f), neg = __float2half(-10000.0f);
     __half h[8];
     if (F32) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(mask) + src));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(mask) + src + 4));
+        const float4 a = __ldca(reinterpret_cast<const float4*>(static_cast<const float*>(mask) + src));
+        const float4 b = __ldca(reinterpret_cast<const float4*>(static_cast<const float*>(mask) + src + 4));
         h[0] = __float2half_rn(a.x); h[1] = __float2half_rn(a.y); h[2] = __float2half_rn(a.z); h[3] = __float2half_rn(a.w);
         h[4] = __float2half_rn(b.x); h[5] = __float2half_rn(b.y); h[6] = __float2half_rn(b.z); h[7] = __float2half_rn(b.w);
     } else {
-        *reinterpret_cast<uint4*>(h) = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(mask) + src));
+        *reinterpret_cast<uint4*>(h) = __ldca(reinterpret_cast<const uint4*>(static_cast<const __half*>(mask) + src));
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) h[i] = __hmul(neg, __hsub(one, h[i]));
@@ -283,7 +283,7 @@ __device__ __forceinline__ uint4 mask_addend8(const void* mask, size_t src) {
 // blockIdx.x - index_blocks, + tile_blocks, ...
 template <bool F32>
 __global__ void __launch_bounds__(FILL_THREADS)
-fill_kernel(const void* __restrict__ mask, int seq_len, int bm, int bn, const unsigned char* cls, const int* full_row_ptr, const int* part_row_ptr,
+fill_kernel(const void* mask, int seq_len, int bm, int bn, const unsigned char* cls, const int* full_row_ptr, const int* part_row_ptr,
             const int* load_row_ptr, int* full_col_idx, int* part_col_idx, int* load_col_idx, __half* part_block_mask, int index_blocks) {
     __shared__ int s_tile[2];                              // block-row and column of the tile in hand
     grid_dependency_wait();

@@ -38,8 +38,11 @@ __device__ __forceinline__ bool elect_one() {
 // ---------------------------------------------------------------------------------
 // Every kernel of the library is launched so that it may become resident while the kernel before it in the stream still runs.
 // It sets itself up (barriers, tensor memory, descriptors), then waits here until that kernel has completed and its writes are
-// visible, and only then reads or writes global memory that a kernel may touch.  EVERY thread block has to come through
-// grid_dependency_wait before it exits: the next kernel's wait covers this one only, and through this one's wait the ones before.
+// visible, and only then reads or writes global memory that a kernel may touch.  Those reads are coherent
+// loads, plain ones or __ldca: __ldg and __restrict__ promise data that stays the same for the whole kernel, which began before it was
+// written, and may be moved ahead of the wait.
+// EVERY thread block has to come through grid_dependency_wait before it exits: the next kernel's wait covers this one only, and
+// through this one's wait the ones before.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Has a kernel reported a failure?  For threads that have come through grid_dependency_wait: before it the kernel that is about to
 // report may still run.  The GEMM kernels ask in their epilogue, under the first products, and write nothing where the answer is yes;

@@ -40,3 +40,15 @@ def test_status_word_is_read_behind_the_dependency_wait(signature, body):
     """Ahead of it the kernel that reports a failure may still run, and the blocks of a cluster may see different words."""
     reads = [m.start() for m in re.finditer(r"\*\s*(?:p\.|report\.)?status\b|failure_reported\(", body)]
     assert all(at > body.index("grid_dependency_wait") for at in reads)
+
+
+@pytest.mark.parametrize("signature,body", dependent_kernels())
+def test_nothing_is_read_as_constant_by_kernels_that_start_early(signature, body):
+    """__ldg, and plain loads through __restrict__ pointers to const, may be moved ahead of the wait: what the kernel ahead writes is not
+    constant for the lifetime of a kernel that starts before it."""
+    assert "__restrict__" not in signature and "__ldg" not in body
+
+
+def test_nothing_is_read_as_constant_by_their_helpers():
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        assert "__ldg(" not in re.sub(r"//[^\n]*", "", open(path).read()), path
