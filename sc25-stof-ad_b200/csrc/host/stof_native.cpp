@@ -80,6 +80,29 @@ void check(int rc, const char* what) {
     if (rc != 0) fail("%s failed (code %d): %s", what, rc, api.last_error());
 }
 
+// The GIL is free while the library launches and torch copies or allocates: where the queue of launches is full they wait for the GPU,
+// and what the GPU waits for may need Python (a host callback in the stream, another thread).
+struct Released {
+    PyThreadState* ts = PyEval_SaveThread();
+    Released() = default;
+    Released(const Released&) = delete;
+    ~Released() { PyEval_RestoreThread(ts); }
+};
+template <class F, class... A>
+void call(const char* what, F* f, A... args) {
+    int rc;
+    {
+        const Released gil;
+        rc = f(args...);
+    }
+    check(rc, what);                         // the error text is the calling thread's own
+}
+at::Tensor packed(const at::Tensor& t) {
+    if (t.is_contiguous()) return t;
+    const Released gil;
+    return t.contiguous();
+}
+
 // ------------------------------------------------------------------------------------------ arguments
 // A tensor argument (nullptr for None); anything else is a TypeError.
 const at::Tensor* tensor_arg(PyObject* o, const char* what) {
@@ -149,7 +172,10 @@ struct Launch {                              // device made current, its current
 };
 
 // A new tensor on t's device, without the dispatcher's round
-at::Tensor make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor& t) { return at::detail::empty_cuda(shape, type, t.device(), std::nullopt); }
+at::Tensor make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor& t) {
+    const Released gil;
+    return at::detail::empty_cuda(shape, type, t.device(), std::nullopt);
+}
 
 // ------------------------------------------------------------------------------------------ matrices
 struct Rows {                                // a (..., C) tensor seen as rows of C with a contiguous last dimension
@@ -169,7 +195,10 @@ Rows as_rows(const at::Tensor& t) {
         r.ptr = t.data_ptr();
         return r;
     }
-    r.keep = (t.stride(d - 1) != 1 ? t.contiguous() : t).reshape({-1, r.cols});
+    {
+        const Released gil;
+        r.keep = (t.stride(d - 1) != 1 ? t.contiguous() : t).reshape({-1, r.cols});
+    }
     r.rows = r.keep.size(0);
     r.ld = r.keep.stride(0);
     r.ptr = r.keep.data_ptr();
@@ -181,7 +210,7 @@ const void* vector_arg(const at::Tensor* v, int64_t n, at::Tensor& keep, const c
     if (v == nullptr) return nullptr;
     if (v->numel() != n || !is_half(*v)) fail("%s", text);
     if (v->is_contiguous()) return v->data_ptr();
-    keep = v->reshape({-1}).contiguous();
+    keep = packed(*v).reshape({-1});
     return keep.data_ptr();
 }
 
@@ -223,7 +252,7 @@ Weight weight_arg(const at::Tensor& w) {
         r.ptr = w.data_ptr();
         r.ld = w.stride(0);
     } else {
-        r.keep = w.contiguous();
+        r.keep = packed(w);
         r.ptr = r.keep.data_ptr();
         r.ld = r.keep.stride(0);
     }
@@ -247,9 +276,8 @@ at::Tensor gemm_core(const Launch& l, const at::Tensor& a, const at::Tensor& w, 
         r = as_rows(*residual);
         if (r.rows != x.rows || r.cols != m.n) fail("gemm: residual must be float16 of the output's shape");
     }
-    check(api.gemm_bias_act(x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, c.ptr, c.ld, static_cast<int>(x.rows), static_cast<int>(m.n),
-                            static_cast<int>(m.k), epilogue, l.status, l.stream),
-          "stof_gemm_bias_act");
+    call("stof_gemm_bias_act", api.gemm_bias_act, x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, c.ptr, c.ld, static_cast<int>(x.rows), static_cast<int>(m.n),
+         static_cast<int>(m.k), epilogue, l.status, l.stream);
     return c.made;
 }
 
@@ -271,9 +299,8 @@ at::Tensor gemm_ln_core(const Launch& l, const at::Tensor& a, const at::Tensor& 
         r = as_rows(*residual);
         if (r.rows != x.rows || r.cols != m.n) fail("gemm+layernorm: residual must be float16 of the output's shape");
     }
-    check(api.gemm_ln(x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), c.ptr, c.ld, static_cast<int>(x.rows),
-                      static_cast<int>(m.n), static_cast<int>(m.k), l.status, l.stream),
-          "stof_gemm_bias_residual_layernorm");
+    call("stof_gemm_bias_residual_layernorm", api.gemm_ln, x.ptr, x.ld, m.ptr, m.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), c.ptr, c.ld,
+         static_cast<int>(x.rows), static_cast<int>(m.n), static_cast<int>(m.k), l.status, l.stream);
     return c.made;
 }
 
@@ -293,9 +320,8 @@ at::Tensor layernorm_core(const Launch& l, const at::Tensor& a, const at::Tensor
     const void* g = vector_arg(gamma, x.cols, kept[1], text);
     const void* t = vector_arg(beta, x.cols, kept[2], text);
     const Out y = output_rows(out, a, x.rows, x.cols, "layernorm");
-    check(api.layernorm(x.ptr, x.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), y.ptr, y.ld, static_cast<int>(x.rows),
-                        static_cast<int>(x.cols), l.status, l.stream),
-          "stof_bias_residual_layernorm");
+    call("stof_bias_residual_layernorm", api.layernorm, x.ptr, x.ld, b, r.ptr, r.ld, g, t, static_cast<float>(eps), y.ptr, y.ld, static_cast<int>(x.rows),
+         static_cast<int>(x.cols), l.status, l.stream);
     return y.made;
 }
 
@@ -387,12 +413,12 @@ void attention_launch(const Launch& l, const PlanEntry& e, const HeadView& q, co
     const int bm = static_cast<int>(e.key.bm), bn = static_cast<int>(e.key.bn);
     const int* prp = static_cast<const int*>(e.index[2].data_ptr());
     const void* pbm = tiles != nullptr ? tiles->data_ptr() : nullptr;
-    const int rc = e.schedule.defined()
-        ? api.block_attn_scheduled(q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride, prp, pbm,
-                                   e.plan.data_ptr(), bm, bn, 4, scale, static_cast<const int*>(e.schedule.data_ptr()), e.blocks, l.status, l.stream)
-        : api.block_attn(q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride, prp, pbm,
-                         e.plan.data_ptr(), bm, bn, 4, scale, l.status, l.stream);
-    check(rc, "stof_block_attn");
+    if (e.schedule.defined())
+        call("stof_block_attn", api.block_attn_scheduled, q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride,
+             prp, pbm, e.plan.data_ptr(), bm, bn, 4, scale, static_cast<const int*>(e.schedule.data_ptr()), e.blocks, l.status, l.stream);
+    else
+        call("stof_block_attn", api.block_attn, q.ptr, k.ptr, v.ptr, out.ptr, B, H, S, head_dim, q.stride, k.stride, v.stride, out.stride, prp, pbm,
+             e.plan.data_ptr(), bm, bn, 4, scale, l.status, l.stream);
 }
 
 Index index_args(PyObject* const* a) {
@@ -491,7 +517,7 @@ PyObject* py_attention_inplace(PyObject*, PyObject* const* a, Py_ssize_t n) {
         need_args(n, 10, "attention_inplace");
         const at::Tensor &q = tensor_needed(a[0], "attention"), &k = tensor_needed(a[1], "attention"), &v = tensor_needed(a[2], "attention");
         if (!q.is_contiguous()) fail("block_attn_mask: q must be contiguous (it is overwritten in place)");
-        const at::Tensor kc = k.contiguous(), vc = v.contiguous();
+        const at::Tensor kc = packed(k), vc = packed(v);
         Index ix;
         at::Tensor kept[5];
         PyObject* made[5] = {};
@@ -503,7 +529,7 @@ PyObject* py_attention_inplace(PyObject*, PyObject* const* a, Py_ssize_t n) {
         for (int i = 0; i < 5; ++i) {
             const at::Tensor& t = tensor_needed(a[3 + i], "block index");
             args[i] = a[3 + i];
-            if (!t.is_contiguous()) args[i] = made[i] = wrap(t.contiguous());
+            if (!t.is_contiguous()) args[i] = made[i] = wrap(packed(t));
         }
         attention_core(q, kc, vc, q, index_args(args), long_arg(a[8]), long_arg(a[9]), -1.0);
         return same(a[0]);
@@ -753,9 +779,8 @@ PyObject* py_sparse_storage(PyObject*, PyObject* const* a, Py_ssize_t n) {
         stof_mask_notice got;
         {
             Notice notice(m.get_device());
-            check(api.mask_classify_notify(m.data_ptr(), dt, static_cast<int>(B), s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(),
-                                           nnz.data_ptr<float>(), ws.data_ptr(), ws_bytes, notice.header(), l.status, notice.record(), notice.stamp, l.stream),
-                  "stof_mask_classify");
+            call("stof_mask_classify", api.mask_classify_notify, m.data_ptr(), dt, static_cast<int>(B), s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(),
+                 lrp.data_ptr<int>(), nnz.data_ptr<float>(), ws.data_ptr(), ws_bytes, notice.header(), l.status, notice.record(), notice.stamp, l.stream);
             got = notice.wait(stream);
         }
         if (got.status != 0) {
@@ -764,11 +789,14 @@ PyObject* py_sparse_storage(PyObject*, PyObject* const* a, Py_ssize_t n) {
             Py_DECREF(r);
         }
         const at::Tensor fci = make({got.n_full}, at::kInt, m), pci = make({got.n_part}, at::kInt, m), lci = make({got.n_full + got.n_part}, at::kInt, m);
-        const at::Tensor tiles = got.n_part > 0 ? make({got.n_part, bm, bn}, at::kHalf, m) : at::ones({1, bm, bn}, m.options().dtype(at::kHalf));
+        at::Tensor tiles = make({got.n_part > 0 ? got.n_part : 1, bm, bn}, at::kHalf, m);
+        if (got.n_part == 0) {
+            const Released gil;
+            tiles.fill_(1);
+        }
         if (got.n_full + got.n_part > 0)
-            check(api.mask_fill(m.data_ptr(), dt, s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(), fci.data_ptr<int>(),
-                                pci.data_ptr<int>(), lci.data_ptr<int>(), got.n_part > 0 ? tiles.data_ptr() : nullptr, ws.data_ptr(), ws_bytes, l.stream),
-                  "stof_mask_fill");
+            call("stof_mask_fill", api.mask_fill, m.data_ptr(), dt, s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(), fci.data_ptr<int>(),
+                 pci.data_ptr<int>(), lci.data_ptr<int>(), got.n_part > 0 ? tiles.data_ptr() : nullptr, ws.data_ptr(), ws_bytes, l.stream);
         const at::Tensor* out[8] = {&nnz, &frp, &fci, &prp, &pci, &tiles, &lrp, &lci};
         PyObject* tuple = PyTuple_New(8);
         for (int i = 0; i < 8; ++i) PyTuple_SET_ITEM(tuple, i, wrap(*out[i]));

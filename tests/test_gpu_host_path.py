@@ -52,3 +52,66 @@ def test_index_checks_hold_for_an_index_whose_plan_is_known():
     for other in (strided, plain.view(torch.float32)):
         with pytest.raises(stof_b200.StofError, match="contiguous int32"):
             stof_b200.block_attention(q, k, v, torch.empty_like(q), frp, fci, other, pci, pbm, lrp, lci, block, block)
+
+
+SLOW_LIBRARY = """
+#include <stddef.h>
+#include <unistd.h>
+const char* stof_last_error(void) { return ""; }
+size_t stof_mask_workspace_bytes(int s, int bm, int bn) { return 4096; }
+int stof_mask_classify_notify() { usleep(200000); return -2; }
+int stof_mask_fill() { usleep(200000); return 0; }
+int stof_block_attn() { usleep(200000); return 0; }
+int stof_block_attn_scheduled() { usleep(200000); return 0; }
+int stof_gemm_bias_act() { usleep(200000); return 0; }
+int stof_gemm_bias_residual_layernorm() { usleep(200000); return 0; }
+int stof_bias_residual_layernorm() { usleep(200000); return 0; }
+"""
+
+
+def test_python_threads_run_while_the_library_is_in_a_call(tmp_path, monkeypatch):
+    """The native path bound to a library whose calls take 0.2 s, as a launch does that finds the queue full: another Python thread gets on."""
+    import subprocess
+    import threading
+    import time
+    import stof_b200
+    from stof_b200 import _lib
+    source, library = tmp_path / "slow.c", tmp_path / "slow.so"
+    source.write_text(SLOW_LIBRARY)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", "-w", "-o", str(library), str(source)])
+    x, w = _rand((8, 64), 1).cuda(), _rand((64, 64), 2).cuda()
+    idx, (q, k, v) = _index(256, 32, 40), (_rand((1, 2, 256, 64), i).cuda() for i in range(3))
+    mask = torch.ones(1, 64, 64, device="cuda")
+    out = torch.empty_like(q)
+    calls = {"gemm": lambda: stof_b200.gemm_bias(x, w), "gemm_ln": lambda: stof_b200.gemm_bias_residual_layernorm(x, w, None, None, None, None, 1e-5),
+             "layernorm": lambda: stof_b200.bias_residual_layernorm(x), "attention": lambda: stof_b200.block_attention(q, k, v, out, *idx, 32, 32),
+             "compaction": lambda: stof_b200.get_sparse_storage(mask, 64, 64)}
+    for f in calls.values():
+        f()
+    ticks, stop = [0], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks[0] += 1
+            time.sleep(0.001)
+
+    other = threading.Thread(target=tick)
+    try:
+        with monkeypatch.context() as patch:
+            patch.setattr(_lib, "_LIB_PATH", str(library))
+            patch.setattr(_lib, "_native", None)
+            _lib.native()
+            other.start()
+            for name, f in calls.items():
+                before = ticks[0]
+                try:
+                    f()
+                except stof_b200.StofError:
+                    assert name == "compaction"              # its stand-in reports a failure, as nothing writes the counts
+                assert ticks[0] - before >= 20, name
+    finally:
+        stop.set()
+        other.join()
+        _lib._native = None
+        _lib.native()
+    assert (stof_b200.gemm_bias(x, w).float() - (x.float() @ w.float())).abs().max() < 0.1
