@@ -572,18 +572,28 @@ PyObject* py_forget(PyObject*, PyObject* arg) {
 }
 
 // ------------------------------------------------------------------------------------------ encoder and decoder stacks
-// A layer's weights, by attribute name, as tensors (the objects stay alive in the layer)
+// A layer's weights, by attribute name, as tensors (the objects stay alive in the layer).  Biases, gamma and beta may be None: an
+// undefined tensor, which `given` turns into the operators' nullptr.
 struct LayerReader {
     PyObject* layer;
-    at::Tensor operator()(PyObject* name) const {
+    at::Tensor vector(PyObject* name) const {
         PyObject* o = PyObject_GetAttr(layer, name);
         if (o == nullptr) throw PythonFail{};
         struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } drop{o};
-        const at::Tensor t = tensor_needed(o, "layer weight");
-        need_cuda(&t);
+        const at::Tensor* t = tensor_arg(o, "layer weight");
+        need_cuda(t);
+        return t != nullptr ? *t : at::Tensor();
+    }
+    at::Tensor operator()(PyObject* name) const {
+        const at::Tensor t = vector(name);
+        if (!t.defined()) {
+            PyErr_Format(PyExc_TypeError, "layer weight %U: a tensor expected, got None", name);
+            throw PythonFail{};
+        }
         return t;
     }
 };
+inline const at::Tensor* given(const at::Tensor& t) { return t.defined() ? &t : nullptr; }
 #define STOF_NAME(s) ([] { static PyObject* n = PyUnicode_InternFromString(s); return n; }())
 
 struct Stack {
@@ -597,7 +607,7 @@ struct Stack {
 };
 
 void attention_sublayer(const Launch& l, const Stack& s, const PlanEntry& plan, const at::Tensor& x, const at::Tensor& wqkv, const at::Tensor& bqkv) {
-    gemm_core(l, x, wqkv, &bqkv, STOF_EPI_BIAS, nullptr, &s.qkv);
+    gemm_core(l, x, wqkv, given(bqkv), STOF_EPI_BIAS, nullptr, &s.qkv);
     const long long S = s.ctx.size(1), hid = s.ctx.size(2), D = hid / s.heads;
     char* base = static_cast<char*>(s.qkv.data_ptr());
     const HeadView q{base, {S * 3 * hid, D, 3 * hid}};
@@ -610,10 +620,10 @@ void attention_sublayer(const Launch& l, const Stack& s, const PlanEntry& plan, 
 void residual_layernorm(const Launch& l, bool fuse, const at::Tensor& a, const at::Tensor& w, const at::Tensor& bias, const at::Tensor& residual,
                         const at::Tensor& g, const at::Tensor& b, double eps, const at::Tensor& out) {
     if (fuse) {
-        gemm_ln_core(l, a, w, &bias, &residual, &g, &b, eps, &out);
+        gemm_ln_core(l, a, w, given(bias), &residual, given(g), given(b), eps, &out);
     } else {
-        gemm_core(l, a, w, &bias, STOF_EPI_BIAS_RESIDUAL, &residual, &out);
-        layernorm_core(l, out, nullptr, nullptr, &g, &b, eps, &out);
+        gemm_core(l, a, w, given(bias), STOF_EPI_BIAS_RESIDUAL, &residual, &out);
+        layernorm_core(l, out, nullptr, nullptr, given(g), given(b), eps, &out);
     }
 }
 
@@ -659,9 +669,9 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
             auto sublayer = [&](PyObject* nqkv, PyObject* nbqkv, PyObject* no, PyObject* nbo, PyObject* ng, PyObject* nb) {
                 // looked up per sublayer: an index used for the first time is planned again, better, at its second use
                 const PlanEntry plan = plan_lookup(s.ix, hidden.size(1), hidden.size(0), s.heads, s.bm, s.bn, hidden.get_device());
-                attention_sublayer(l, s, plan, x, w(nqkv), w(nbqkv));
+                attention_sublayer(l, s, plan, x, w(nqkv), w.vector(nbqkv));
                 const at::Tensor& out = s.y[yi];
-                residual_layernorm(l, fuse, s.ctx, w(no), w(nbo), x, w(ng), w(nb), s.eps, out);
+                residual_layernorm(l, fuse, s.ctx, w(no), w.vector(nbo), x, w.vector(ng), w.vector(nb), s.eps, out);
                 x = out;
                 x_obj = s.y_obj[yi];
                 yi = (yi + 1) % s.n_y;
@@ -672,10 +682,11 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
             } else {
                 sublayer(STOF_NAME("Wqkv"), STOF_NAME("bqkv"), STOF_NAME("Wo"), STOF_NAME("bo"), STOF_NAME("g1"), STOF_NAME("b1"));
             }
-            const at::Tensor bi1 = w(STOF_NAME("bi1"));
-            gemm_core(l, x, w(STOF_NAME("W1")), &bi1, act, nullptr, &s.inter);
+            const at::Tensor bi1 = w.vector(STOF_NAME("bi1"));
+            gemm_core(l, x, w(STOF_NAME("W1")), given(bi1), act, nullptr, &s.inter);
             const at::Tensor& out = s.y[yi];
-            residual_layernorm(l, fuse, s.inter, w(STOF_NAME("W2")), w(STOF_NAME("bi2")), x, w(STOF_NAME("g2")), w(STOF_NAME("b2")), s.eps, out);
+            residual_layernorm(l, fuse, s.inter, w(STOF_NAME("W2")), w.vector(STOF_NAME("bi2")), x, w.vector(STOF_NAME("g2")), w.vector(STOF_NAME("b2")),
+                               s.eps, out);
             x = out;
             x_obj = s.y_obj[yi];
             yi = (yi + 1) % s.n_y;

@@ -115,3 +115,22 @@ def test_python_threads_run_while_the_library_is_in_a_call(tmp_path, monkeypatch
         _lib._native = None
         _lib.native()
     assert (stof_b200.gemm_bias(x, w).float() - (x.float() @ w.float())).abs().max() < 0.1
+
+
+@pytest.mark.parametrize("fuse", [True, False])
+def test_stack_without_biases_and_affine(fuse):
+    """Layers whose bias, gamma and beta are None (T5 has no biases) give what zeros and ones give."""
+    from stof_b200 import EncoderWeights
+    hid, x = 128, _rand((2, 64, 128), 5).cuda()
+    names = ("bqkv", "bo", "bi1", "bi2", "g1", "b1", "g2", "b2")
+    enc, same = _encoder(hid, 2, 256, 64, without=names), _encoder(hid, 2, 256, 64)
+    enc.fuse_layernorm = same.fuse_layernorm = fuse
+    w = {k: getattr(enc.layers[0], k) for k in EncoderWeights.__dataclass_fields__}
+    for name in names:
+        w[name] = torch.full_like(getattr(same.layers[0], name), 1.0 if name[0] == "g" else 0.0)
+    same.layers = [EncoderWeights(**w)]
+    assert torch.equal(enc(x), same(x))
+    w["Wo"] = None
+    same.layers = [EncoderWeights(**w)]
+    with pytest.raises(TypeError, match="Wo"):
+        same(x)
