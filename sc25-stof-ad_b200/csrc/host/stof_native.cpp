@@ -23,6 +23,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -440,7 +441,7 @@ HeadView head_view(const at::Tensor& t) {
 }
 
 void attention_core(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out, const Index& ix, int64_t bm, int64_t bn,
-                    double scale) {
+                    std::optional<double> softmax_scale = std::nullopt) {
     const at::Tensor* all[4] = {&q, &k, &v, &out};
     for (const at::Tensor* t : all) need_cuda(t);
     for (const at::Tensor* t : all)
@@ -451,7 +452,7 @@ void attention_core(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
         if (t->stride(3) != 1) fail("block attention: the head dimension must be contiguous");
     }
     if (bm <= 0 || bn <= 0) fail("block attention: block sizes must be positive");
-    if (scale < 0) scale = 1.0 / std::sqrt(static_cast<double>(q.size(3)));          // src/ops/src/block_attn_mask.cpp:32
+    const double scale = softmax_scale ? *softmax_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));          // src/ops/src/block_attn_mask.cpp:32
     const Launch l(q);
     const PlanEntry e = plan_lookup(ix, q.size(2), q.size(0), q.size(1), bm, bn, q.get_device());
     attention_launch(l, e, head_view(q), head_view(k), head_view(v), head_view(out), ix.tiles, static_cast<int>(q.size(3)),
@@ -501,12 +502,13 @@ PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, block_m, block_n, scale) -> out;
-// a negative scale stands for 1 / sqrt(head_dim)
+// None as scale stands for 1 / sqrt(head_dim)
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         need_args(n, 12, "attention");
         attention_core(tensor_needed(a[0], "attention"), tensor_needed(a[1], "attention"), tensor_needed(a[2], "attention"),
-                       tensor_needed(a[3], "attention"), index_args(a + 4), long_arg(a[9]), long_arg(a[10]), double_arg(a[11]));
+                       tensor_needed(a[3], "attention"), index_args(a + 4), long_arg(a[9]), long_arg(a[10]),
+                       a[11] != Py_None ? std::optional<double>(double_arg(a[11])) : std::nullopt);
         return same(a[3]);
     });
 }
@@ -531,7 +533,7 @@ PyObject* py_attention_inplace(PyObject*, PyObject* const* a, Py_ssize_t n) {
             args[i] = a[3 + i];
             if (!t.is_contiguous()) args[i] = made[i] = wrap(packed(t));
         }
-        attention_core(q, kc, vc, q, index_args(args), long_arg(a[8]), long_arg(a[9]), -1.0);
+        attention_core(q, kc, vc, q, index_args(args), long_arg(a[8]), long_arg(a[9]));
         return same(a[0]);
     });
 }
@@ -552,7 +554,7 @@ PyObject* py_merged_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
             fail("row-wise attention: result must be a contiguous (batch, S, heads*64) tensor");
         }
         const at::Tensor& r = result != nullptr ? *result : made;
-        attention_core(q, k, v, r.as_strided({B, H, S, D}, {S * H * D, D, H * D, 1}), index_args(a + 4), long_arg(a[9]), long_arg(a[10]), -1.0);
+        attention_core(q, k, v, r.as_strided({B, H, S, D}, {S * H * D, D, H * D, 1}), index_args(a + 4), long_arg(a[9]), long_arg(a[10]));
         return result != nullptr ? same(a[3]) : wrap(made);
     });
 }

@@ -253,7 +253,7 @@ def block_attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part
     `load_row_ptr` / `load_col_idx` are accepted for signature compatibility (they are the merge of
     the full and partial lists, which is what the kernel's plan is built from)."""
     return (_lib._native or _lib.native()).attention(q, k, v, out, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,
-                                                     block_m, block_n, -1.0 if softmax_scale is None else softmax_scale)
+                                                     block_m, block_n, softmax_scale)
 
 
 def block_attn_mask(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask,

@@ -134,3 +134,13 @@ def test_stack_without_biases_and_affine(fuse):
     same.layers = [EncoderWeights(**w)]
     with pytest.raises(TypeError, match="Wo"):
         same(x)
+
+
+def test_softmax_scale_has_to_be_positive():
+    import stof_b200
+    idx, (q, k, v) = _index(256, 32, 40), (_rand((1, 2, 256, 64), i).cuda() for i in range(3))
+    for scale in (-0.125, -1.0, 0.0, float("nan")):
+        with pytest.raises(stof_b200.StofError, match="positive"):
+            stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32, softmax_scale=scale)
+    default = stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32)
+    assert torch.equal(stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32, softmax_scale=0.125), default)
