@@ -122,8 +122,12 @@ const at::Tensor& tensor_needed(PyObject* o, const char* what) {
     }
     return *t;
 }
+// a whole number as int(o) gives it, for what is not an int itself (a size that was computed as a float)
 long long_arg(PyObject* o) {
-    const long v = PyLong_AsLong(o);
+    PyObject* whole = PyLong_Check(o) ? o : PyNumber_Long(o);
+    if (whole == nullptr) throw PythonFail{};
+    const long v = PyLong_AsLong(whole);
+    if (whole != o) Py_DECREF(whole);
     if (v == -1 && PyErr_Occurred()) throw PythonFail{};
     return v;
 }

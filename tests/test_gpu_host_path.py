@@ -144,3 +144,13 @@ def test_softmax_scale_has_to_be_positive():
             stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32, softmax_scale=scale)
     default = stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32)
     assert torch.equal(stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32, softmax_scale=0.125), default)
+
+
+def test_block_sizes_that_are_whole_but_no_ints():
+    import stof_b200
+    idx, (q, k, v) = _index(256, 32, 40), (_rand((1, 2, 256, 64), i).cuda() for i in range(3))
+    for _ in range(2):                                   # the second use may pair the halves anew, which changes the order of the sums
+        want = stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, 32, 32)
+    for size in (32.0, np.float64(32), np.int64(32), torch.tensor(32)):
+        assert torch.equal(stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, size, size), want)
+        assert torch.equal(stof_b200.block_attn_mask(q.clone(), k, v, *idx, size, size, 4), want)
