@@ -362,6 +362,7 @@ struct Index {
 };
 
 PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads, int64_t bm, int64_t bn, int64_t dev) {
+    if (bm <= 0 || bn <= 0) fail("block attention: block sizes must be positive");
     // On every call, known index or not: base[:n] and base[::2] of one tensor agree in all that the key holds
     for (int i = 0; i < 4; ++i)
         if (ix.t[i]->scalar_type() != at::kInt || !ix.t[i]->is_contiguous()) fail("block attention: index tensors must be contiguous int32");
@@ -455,7 +456,6 @@ void attention_core(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
         if (t->sizes() != q.sizes()) fail("block attention: q, k, v and out must share one (B,H,S,D) shape");
         if (t->stride(3) != 1) fail("block attention: the head dimension must be contiguous");
     }
-    if (bm <= 0 || bn <= 0) fail("block attention: block sizes must be positive");
     const double scale = softmax_scale ? *softmax_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));          // src/ops/src/block_attn_mask.cpp:32
     const Launch l(q);
     const PlanEntry e = plan_lookup(ix, q.size(2), q.size(0), q.size(1), bm, bn, q.get_device());
@@ -646,7 +646,8 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
         s.ctx = tensor_needed(a[3], "ctx");
         s.inter = tensor_needed(a[4], "inter");
         s.n_y = static_cast<int>(PyTuple_GET_SIZE(a[5]));
-        for (int i = 0; i < s.n_y && i < 4; ++i) {
+        if (s.n_y < 1 || s.n_y > 4) fail("encoder: one to four hidden-state buffers expected, got %d", s.n_y);
+        for (int i = 0; i < s.n_y; ++i) {
             s.y_obj[i] = PyTuple_GET_ITEM(a[5], i);
             s.y[i] = tensor_needed(s.y_obj[i], "y");
         }

@@ -154,3 +154,23 @@ def test_block_sizes_that_are_whole_but_no_ints():
     for size in (32.0, np.float64(32), np.int64(32), torch.tensor(32)):
         assert torch.equal(stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx, size, size), want)
         assert torch.equal(stof_b200.block_attn_mask(q.clone(), k, v, *idx, size, size, 4), want)
+
+
+@pytest.mark.parametrize("block_m,block_n", [(0, 32), (32, 0), (-32, 32)])
+def test_stack_refuses_block_sizes_that_are_not_positive(block_m, block_n):
+    """An index that the caller sets comes with block sizes that no compaction has looked at."""
+    import stof_b200
+    enc = _encoder(128, 2, 64, 64)
+    enc.block_m, enc.block_n = block_m, block_n
+    with pytest.raises(stof_b200.StofError, match="positive"):
+        enc(_rand((1, 64, 128), 1).cuda())
+
+
+def test_stack_refuses_more_state_buffers_than_it_rotates():
+    import stof_b200
+    enc = _encoder(128, 2, 64, 64)
+    for count in (0, 5):
+        enc._STATES = count
+        enc._io.clear()
+        with pytest.raises(stof_b200.StofError, match="buffers"):
+            enc(_rand((1, 64, 128), 1).cuda())
