@@ -427,13 +427,13 @@ void attention_launch(const Launch& l, const PlanEntry& e, const HeadView& q, co
              e.plan.data_ptr(), bm, bn, 4, scale, l.status, l.stream);
 }
 
-Index index_args(PyObject* const* a) {
+Index index_args(PyObject* const* a, const at::Tensor* tiles = nullptr) {
     Index ix;
     for (int i = 0; i < 4; ++i) {
         ix.o[i] = a[i];
         ix.t[i] = &tensor_needed(a[i], "block index");
     }
-    ix.tiles = tensor_arg(a[4], "part_block_mask");
+    ix.tiles = tiles != nullptr ? tiles : tensor_arg(a[4], "part_block_mask");
     need_cuda(ix.t[0]);
     need_cuda(ix.t[2]);
     if (ix.tiles != nullptr && (!is_half(*ix.tiles) || !ix.tiles->is_contiguous()))
@@ -523,21 +523,8 @@ PyObject* py_attention_inplace(PyObject*, PyObject* const* a, Py_ssize_t n) {
         need_args(n, 10, "attention_inplace");
         const at::Tensor &q = tensor_needed(a[0], "attention"), &k = tensor_needed(a[1], "attention"), &v = tensor_needed(a[2], "attention");
         if (!q.is_contiguous()) fail("block_attn_mask: q must be contiguous (it is overwritten in place)");
-        const at::Tensor kc = packed(k), vc = packed(v);
-        Index ix;
-        at::Tensor kept[5];
-        PyObject* made[5] = {};
-        struct Release {
-            PyObject** p;
-            ~Release() { for (int i = 0; i < 5; ++i) Py_XDECREF(p[i]); }
-        } release{made};
-        PyObject* args[5];
-        for (int i = 0; i < 5; ++i) {
-            const at::Tensor& t = tensor_needed(a[3 + i], "block index");
-            args[i] = a[3 + i];
-            if (!t.is_contiguous()) args[i] = made[i] = wrap(packed(t));
-        }
-        attention_core(q, kc, vc, q, index_args(args), long_arg(a[8]), long_arg(a[9]));
+        const at::Tensor kc = packed(k), vc = packed(v), tiles = packed(tensor_needed(a[7], "block index"));
+        attention_core(q, kc, vc, q, index_args(a + 3, &tiles), long_arg(a[8]), long_arg(a[9]));
         return same(a[0]);
     });
 }

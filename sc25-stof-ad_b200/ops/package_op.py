@@ -87,5 +87,5 @@ def block_attn_mask_op(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_c
     if _differentiating(q, k, v):
         return Block_Attn_Mask.apply(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, load_row_ptr,
                                      load_col_idx, BLOCK_M, BLOCK_N, num_warps)
-    return _block_attn_mask_forward(q, k, v, full_row_ptr, full_col_idx, part_row_ptr, part_col_idx, part_block_mask, load_row_ptr,
-                                    load_col_idx, BLOCK_M, BLOCK_N, num_warps)
+    return _block_attn_mask_forward(q, k, v, full_row_ptr.contiguous(), full_col_idx.contiguous(), part_row_ptr.contiguous(), part_col_idx.contiguous(),
+                                    part_block_mask, load_row_ptr, load_col_idx, BLOCK_M, BLOCK_N, num_warps)

@@ -174,3 +174,17 @@ def test_stack_refuses_more_state_buffers_than_it_rotates():
         enc._io.clear()
         with pytest.raises(stof_b200.StofError, match="buffers"):
             enc(_rand((1, 64, 128), 1).cuda())
+
+
+def test_strided_index_is_refused_by_the_function_and_packed_by_the_operator():
+    import stof_b200
+    from ops.package_op import block_attn_mask_op
+    idx, (q, k, v) = _index(256, 32, 40), (_rand((1, 2, 256, 64), i).cuda() for i in range(3))
+    want = stof_b200.block_attn_mask(q.clone(), k, v, *idx, 32, 32, 4)
+    strided = tuple(torch.stack((t, t), -1)[..., 0] for t in idx)
+    assert not any(t.is_contiguous() for t in strided)
+    with pytest.raises(stof_b200.StofError, match="contiguous int32"):
+        stof_b200.block_attn_mask(q.clone(), k, v, *strided, 32, 32, 4)
+    tiles = idx[:4] + strided[4:5] + idx[5:]
+    assert (stof_b200.block_attn_mask(q.clone(), k, v, *tiles, 32, 32, 4).float() - want.float()).abs().max() <= 2e-3      # the plan is decided at its second use
+    assert (block_attn_mask_op(q.clone(), k, v, *strided, 32, 32, 4).float() - want.float()).abs().max() <= 2e-3
