@@ -304,7 +304,7 @@ def test_encoder_forward_captured_in_a_cuda_graph():
     _lib.check_status(x.device, "graph replay")
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 8, 2048), (63, 72, 200), (65, 136, 2056), (100, 768, 3000), (130, 712, 4104), (512, 2304, 72), (1000, 2312, 128), (257, 128, 8192)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 2048), (63, 72, 200), (65, 136, 2056), (100, 768, 3000), (130, 712, 4104), (512, 2304, 72), (1000, 2296, 136), (257, 128, 8192)])
 def test_gemm_with_few_tiles_every_epilogue(m, n, k):
     """Shapes that run on the small-tile kernel: 64 x 64, 128 x 64 and 128 x 128 tiles with ragged edges, K not a multiple of the
     stage, K in one, two and four parts over a cluster (from 2048 and 4096 on), in-place residual.  fp16 output of fp32 sums."""
@@ -333,10 +333,12 @@ def test_small_layernorm_epilogue(m, n, k):
     assert _err(got, want) <= 2e-3 * max(1.0, want.abs().max().item())
 
 
-@pytest.mark.parametrize("m,n,k,ldc", [(9601, 256, 64, 256), (4353, 512, 200, 520), (5633, 768, 72, 784), (8065, 1024, 136, 1024), (3841, 1024, 2048, 1032)])
+@pytest.mark.parametrize("m,n,k,ldc", [(9601, 256, 64, 256), (4353, 512, 200, 520), (5633, 768, 72, 784), (8065, 1024, 136, 1024), (3841, 1024, 2048, 1032),
+                                       (8321, 1024, 1032, 1024), (8193, 768, 3080, 768)])
 def test_layernorm_epilogue_over_pairs_of_blocks(m, n, k, ldc):
     """GEMM + LayerNorm beyond what runs at once on small tiles: clusters of 2, 4, 6 and 8 thread blocks, one to three 256-row blocks
-    each, a last one of one row, K not a multiple of the stage, row strides beyond the row, in place over the residual."""
+    each, a last one of one row, K not a multiple of the stage and long enough for the ring of stages to go round several times, row
+    strides beyond the row, in place over the residual."""
     import stof_b200
     a, w, b, r = _rand((m, k), 71), _rand((k, n), 72, k ** -0.5), _rand((n,), 73), _rand((m, n), 74)
     gam, bet = (_rand((n,), 75, 0.3).float() + 1).half(), _rand((n,), 76, 0.3)
@@ -427,3 +429,29 @@ def test_gemms_write_nothing_once_a_failure_is_reported(m, n, k, norm):
     finally:
         word.zero_()
     assert torch.equal(call(out), want)
+
+
+@pytest.mark.parametrize("m,n,k,norm,kernel", [
+    (65, 136, 2056, False, "gemm_split_kernel<3, 64, 64>"), (512, 2304, 72, False, "gemm_split_kernel<3, 128, 64>"),
+    (1000, 2296, 136, False, "gemm_split_kernel<3, 128, 128>"), (1000, 2312, 128, False, "gemm_kernel<3>"), (4096, 2560, 1032, False, "gemm_pair_kernel<3>"),
+    (65, 768, 136, True, "gemm_split_ln_kernel<64, 64>"), (1100, 256, 64, True, "gemm_split_ln_kernel<64, 64>"),
+    (600, 768, 768, True, "gemm_split_ln_kernel<64, 128>"), (2048, 1024, 1024, True, "gemm_ln_kernel"), (3841, 1024, 2048, True, "gemm_ln_kernel"),
+    (8321, 1024, 1032, True, "gemm_ln_kernel"), (8193, 768, 3080, True, "gemm_ln_kernel"), (6144, 768, 3072, True, "layernorm_kernel<3, 2>")])
+def test_shapes_run_on_the_kernels_that_the_tests_take_them_for(m, n, k, norm, kernel):
+    """The dispatch by size, at shapes of the tests above: a rule that moves must not leave a kernel without its comparison.  (148 SMs;
+    with the residual epilogue.)"""
+    import stof_b200
+    from torch.profiler import ProfilerActivity, profile
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148 or "STOF_B200_GEMM_LN" in os.environ or "STOF_B200_GEMM_PAIR" in os.environ:
+        pytest.skip("the sizes are those of 148 SMs and the default dispatch")
+    a, w, r = (torch.zeros(*s, dtype=torch.float16, device="cuda") for s in ((m, k), (k, n), (m, n)))
+    call = (lambda: stof_b200.gemm_bias_residual_layernorm(a, w, None, r, None, None, 1e-5)) if norm else (lambda: stof_b200.gemm_bias_residual(a, w, None, r))
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as record:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in record.events() if "stof::" in e.name]
+    if not names:
+        pytest.skip("the profiler records no kernels here")
+    assert kernel in names[-1], names
