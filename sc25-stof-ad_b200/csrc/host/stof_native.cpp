@@ -19,6 +19,7 @@
 #include <sched.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -381,7 +382,7 @@ PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads
     if (keyed)
         for (size_t i = 0; i < all.size(); ++i)
             if (all[i].key == key) {
-                if (i > 0) std::swap(all[i], all[0]);
+                if (i > 0) std::rotate(all.begin(), all.begin() + static_cast<long>(i), all.begin() + static_cast<long>(i) + 1);
                 return all[0];
             }
     PyObject* r = PyObject_CallFunction(g_plan_for_call, "OOOOLLLLL", ix.o[0], ix.o[1], ix.o[2], ix.o[3], static_cast<long long>(seq),

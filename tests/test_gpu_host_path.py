@@ -188,3 +188,32 @@ def test_strided_index_is_refused_by_the_function_and_packed_by_the_operator():
     tiles = idx[:4] + strided[4:5] + idx[5:]
     assert (stof_b200.block_attn_mask(q.clone(), k, v, *tiles, 32, 32, 4).float() - want.float()).abs().max() <= 2e-3      # the plan is decided at its second use
     assert (block_attn_mask_op(q.clone(), k, v, *strided, 32, 32, 4).float() - want.float()).abs().max() <= 2e-3
+
+
+def test_plan_list_gives_up_the_index_used_longest_ago(monkeypatch):
+    """32 plans are remembered: a 33rd index takes the place of the one that was used longest ago, in whatever order the others were."""
+    import stof_b200
+    from stof_b200 import _lib, attention
+    asked = []
+    counting = lambda *a: asked.append(a[0].data_ptr()) or attention.plan_for_call(*a)
+    q, k, v = (_rand((1, 1, 128, 64), i).cuda() for i in range(3))
+    idx = [_index(128, 64, 200) for _ in range(33)]
+    use = lambda i: stof_b200.block_attention(q, k, v, torch.empty_like(q), *idx[i], 64, 64)
+    device = lambda n: torch.device("cuda", n)
+    native = _lib.native()
+    try:
+        native.bind(_lib._LIB_PATH, _lib.StofError, lambda n: _lib.status_word(device(n)), lambda n, what: _lib.check_status(device(n), what), counting)
+        for i in range(32):
+            use(i), use(i)                               # decided at the second use
+        asked.clear()
+        use(0)                                           # the oldest comes to the front
+        use(32), use(32)                                 # and 1 goes
+        asked.clear()
+        for i in (31, 0, 2):
+            use(i)
+        assert not asked
+        use(1)
+        assert asked == [idx[1][0].data_ptr()]
+    finally:
+        _lib._native = None
+        _lib.native()
