@@ -195,11 +195,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void remote_arrive(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same for an arrive that publishes no memory (an accumulator that has been read): at cluster scope the release waits for the
-// thread's earlier global and remote stores, 1300 cycles in an epilogue
 __device__ __forceinline__ void remote_arrive_cta(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

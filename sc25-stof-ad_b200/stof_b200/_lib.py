@@ -114,12 +114,6 @@ def current_stream_ptr(device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
-def require_cuda(*tensors):
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise StofError("stof_b200 operators need CUDA tensors (there is no CPU fallback)")
-
-
 _status = {}
 
 
