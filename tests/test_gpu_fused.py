@@ -455,3 +455,28 @@ def test_shapes_run_on_the_kernels_that_the_tests_take_them_for(m, n, k, norm, k
     if not names:
         pytest.skip("the profiler records no kernels here")
     assert kernel in names[-1], names
+
+
+@pytest.mark.parametrize("name", ["gemm", "gemm_ln", "attention"])
+def test_operator_as_the_first_cuda_call_of_a_thread(name):
+    """A thread that has made no runtime call yet is bound to no device; the operators that describe their operands to the driver work there."""
+    import threading
+    import stof_b200
+    x, w, q = _rand((64, 64), 1).cuda(), _rand((64, 256), 2).cuda(), _rand((1, 1, 128, 64), 3).cuda()
+    index, y, o = stof_b200.get_sparse_storage(torch.ones(1, 128, 128, device="cuda"), 64, 64)[1:], torch.empty(64, 256).half().cuda(), torch.empty_like(q)
+    calls = {"gemm": lambda: stof_b200.gemm_bias(x, w, out=y), "gemm_ln": lambda: stof_b200.gemm_bias_residual_layernorm(x, w, None, None, None, None, 1e-5, out=y),
+             "attention": lambda: stof_b200.block_attention(q, q, q, o, *index, 64, 64)}
+    for _ in range(2):
+        calls[name]()
+    failed = []
+
+    def first():
+        try:
+            calls[name]()
+        except Exception as error:
+            failed.append(repr(error))
+
+    thread = threading.Thread(target=first)
+    thread.start()
+    thread.join()
+    assert not failed, failed
