@@ -83,12 +83,14 @@ void check(int rc, const char* what) {
 }
 
 // The GIL is free while the library launches and torch copies or allocates: where the queue of launches is full they wait for the GPU,
-// and what the GPU waits for may need Python (a host callback in the stream, another thread).
+// and what the GPU waits for may need Python (a host callback in the stream, another thread).  One that stands inside another does
+// nothing; whoever needs several calls in a row takes it once around them, as every turn with the lock may have to wait for a thread
+// that computes in Python.
 struct Released {
-    PyThreadState* ts = PyEval_SaveThread();
+    PyThreadState* ts = PyGILState_Check() ? PyEval_SaveThread() : nullptr;
     Released() = default;
     Released(const Released&) = delete;
-    ~Released() { PyEval_RestoreThread(ts); }
+    ~Released() { if (ts != nullptr) PyEval_RestoreThread(ts); }
 };
 template <class F, class... A>
 void call(const char* what, F* f, A... args) {
@@ -349,6 +351,7 @@ struct PlanEntry {
     PlanKey key;
     at::Tensor index[4], plan, schedule;     // schedule: undefined when the default deal is used
     int blocks;
+    bool decided;                            // remembered: a later lookup gives the same
 };
 constexpr size_t MAX_PLANS = 32;
 std::vector<PlanEntry>& plans() {
@@ -401,8 +404,9 @@ PlanEntry plan_lookup(const Index& ix, int64_t seq, int64_t batch, int64_t heads
     e.plan = tensor_needed(plan, "plan");
     if (schedule != Py_None) e.schedule = tensor_needed(schedule, "schedule");
     e.blocks = blocks;
+    e.decided = keyed && final_;
     Py_DECREF(r);
-    if (keyed && final_) {
+    if (e.decided) {
         if (all.size() >= MAX_PLANS) all.pop_back();
         all.insert(all.begin(), e);
     }
@@ -650,41 +654,63 @@ PyObject* py_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
             fail("encoder: hidden size %lld is not a multiple of the %lld heads", static_cast<long long>(hid), static_cast<long long>(s.heads));
         const int act = static_cast<int>(long_arg(a[15]));
         const bool fuse = PyObject_IsTrue(a[16]) == 1, decoder = PyObject_IsTrue(a[17]) == 1;
-        const Launch l(hidden);
-        at::Tensor x = hidden;
-        PyObject* x_obj = a[1];
-        int yi = 0;
-        const Py_ssize_t layers = PySequence_Size(a[0]);
-        if (layers < 0) throw PythonFail{};
-        for (Py_ssize_t i = 0; i < layers; ++i) {
+        struct Attention { at::Tensor Wqkv, bqkv, Wo, bo, g, b; };
+        struct Layer { Attention a[2]; at::Tensor W1, bi1, W2, bi2, g2, b2; };
+        const Py_ssize_t count = PySequence_Size(a[0]);
+        if (count < 0) throw PythonFail{};
+        std::vector<Layer> layers(static_cast<size_t>(count));
+        for (Py_ssize_t i = 0; i < count; ++i) {
             PyObject* layer = PySequence_GetItem(a[0], i);
             if (layer == nullptr) throw PythonFail{};
             struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } drop{layer};
             const LayerReader w{layer};
-            auto sublayer = [&](PyObject* nqkv, PyObject* nbqkv, PyObject* no, PyObject* nbo, PyObject* ng, PyObject* nb) {
-                // looked up per sublayer: an index used for the first time is planned again, better, at its second use
-                const PlanEntry plan = plan_lookup(s.ix, hidden.size(1), hidden.size(0), s.heads, s.bm, s.bn, hidden.get_device());
-                attention_sublayer(l, s, plan, x, w(nqkv), w.vector(nbqkv));
-                const at::Tensor& out = s.y[yi];
-                residual_layernorm(l, fuse, s.ctx, w(no), w.vector(nbo), x, w.vector(ng), w.vector(nb), s.eps, out);
-                x = out;
-                x_obj = s.y_obj[yi];
-                yi = (yi + 1) % s.n_y;
-            };
+            Layer& m = layers[static_cast<size_t>(i)];
             if (decoder) {
-                sublayer(STOF_NAME("Wqkv_a"), STOF_NAME("bqkv_a"), STOF_NAME("Wo_a"), STOF_NAME("bo_a"), STOF_NAME("g_a"), STOF_NAME("b_a"));
-                sublayer(STOF_NAME("Wqkv_c"), STOF_NAME("bqkv_c"), STOF_NAME("Wo_c"), STOF_NAME("bo_c"), STOF_NAME("g_c"), STOF_NAME("b_c"));
+                m.a[0] = {w(STOF_NAME("Wqkv_a")), w.vector(STOF_NAME("bqkv_a")), w(STOF_NAME("Wo_a")), w.vector(STOF_NAME("bo_a")), w.vector(STOF_NAME("g_a")),
+                          w.vector(STOF_NAME("b_a"))};
+                m.a[1] = {w(STOF_NAME("Wqkv_c")), w.vector(STOF_NAME("bqkv_c")), w(STOF_NAME("Wo_c")), w.vector(STOF_NAME("bo_c")), w.vector(STOF_NAME("g_c")),
+                          w.vector(STOF_NAME("b_c"))};
             } else {
-                sublayer(STOF_NAME("Wqkv"), STOF_NAME("bqkv"), STOF_NAME("Wo"), STOF_NAME("bo"), STOF_NAME("g1"), STOF_NAME("b1"));
+                m.a[0] = {w(STOF_NAME("Wqkv")), w.vector(STOF_NAME("bqkv")), w(STOF_NAME("Wo")), w.vector(STOF_NAME("bo")), w.vector(STOF_NAME("g1")),
+                          w.vector(STOF_NAME("b1"))};
             }
-            const at::Tensor bi1 = w.vector(STOF_NAME("bi1"));
-            gemm_core(l, x, w(STOF_NAME("W1")), given(bi1), act, nullptr, &s.inter);
-            const at::Tensor& out = s.y[yi];
-            residual_layernorm(l, fuse, s.inter, w(STOF_NAME("W2")), w.vector(STOF_NAME("bi2")), x, w.vector(STOF_NAME("g2")), w.vector(STOF_NAME("b2")),
-                               s.eps, out);
-            x = out;
+            m.W1 = w(STOF_NAME("W1"));
+            m.bi1 = w.vector(STOF_NAME("bi1"));
+            m.W2 = w(STOF_NAME("W2"));
+            m.bi2 = w.vector(STOF_NAME("bi2"));
+            m.g2 = w.vector(STOF_NAME("g2"));
+            m.b2 = w.vector(STOF_NAME("b2"));
+        }
+        const Launch l(hidden);
+        at::Tensor x = hidden;
+        PyObject* x_obj = a[1];
+        int yi = 0;
+        auto next_state = [&] {
+            x = s.y[yi];
             x_obj = s.y_obj[yi];
             yi = (yi + 1) % s.n_y;
+        };
+        {
+            // an index used for the first time is planned again, better, at its second use: looked up until that is done, and from
+            // there on nothing needs Python
+            PlanEntry plan;
+            plan.decided = false;
+            std::optional<Released> gil;
+            for (const Layer& m : layers) {
+                for (int i = 0; i < (decoder ? 2 : 1); ++i) {
+                    if (!gil) {
+                        plan = plan_lookup(s.ix, hidden.size(1), hidden.size(0), s.heads, s.bm, s.bn, hidden.get_device());
+                        if (plan.decided) gil.emplace();
+                    }
+                    const Attention& w = m.a[i];
+                    attention_sublayer(l, s, plan, x, w.Wqkv, w.bqkv);
+                    residual_layernorm(l, fuse, s.ctx, w.Wo, w.bo, x, w.g, w.b, s.eps, s.y[yi]);
+                    next_state();
+                }
+                gemm_core(l, x, m.W1, given(m.bi1), act, nullptr, &s.inter);
+                residual_layernorm(l, fuse, s.inter, m.W2, m.bi2, x, m.g2, m.b2, s.eps, s.y[yi]);
+                next_state();
+            }
         }
         return same(x_obj);
     });
@@ -726,9 +752,8 @@ struct Notice {
             for (int i = 0; i < NOTICES && slot < 0; ++i)
                 if (!pool.busy[i]) slot = i;
             if (slot < 0) {                  // sixteen other threads are waiting for theirs
-                PyThreadState* ts = PyEval_SaveThread();
+                const Released gil;
                 sched_yield();
-                PyEval_RestoreThread(ts);
             }
         }
         pool.busy[slot] = true;
@@ -742,7 +767,7 @@ struct Notice {
     stof_mask_notice wait(cudaStream_t stream) {
         volatile unsigned long long* at = &record()->stamp;
         cudaError_t e = cudaErrorNotReady;
-        PyThreadState* ts = PyEval_SaveThread();
+        const Released gil;
         for (unsigned spins = 1; *at != stamp; ++spins) {
             if ((spins & 0x3FFF) != 0) {
                 __builtin_ia32_pause();
@@ -751,7 +776,6 @@ struct Notice {
             e = cudaStreamQuery(stream);
             if (e != cudaErrorNotReady) break;
         }
-        PyEval_RestoreThread(ts);
         if (*at != stamp) {
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (*at != stamp) fail("get_sparse_storage: the compaction did not report: %s", cudaGetErrorString(e));
@@ -778,13 +802,17 @@ PyObject* py_sparse_storage(PyObject*, PyObject* const* a, Py_ssize_t n) {
         cuda_ok(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing");
         if (capturing != cudaStreamCaptureStatusNone) fail("get_sparse_storage: the sizes of its outputs depend on the data, so it cannot be captured");
         const int64_t rows = S / bm + 1;
-        const at::Tensor frp = make({rows}, at::kInt, m), prp = make({rows}, at::kInt, m), lrp = make({rows}, at::kInt, m);
-        const at::Tensor nnz = make({}, at::kFloat, m);
         const size_t ws_bytes = api.mask_workspace_bytes(s, ibm, ibn);
-        const at::Tensor ws = make({static_cast<int64_t>(ws_bytes)}, at::kByte, m);
+        at::Tensor frp, prp, lrp, nnz, ws, fci, pci, lci, tiles;
         stof_mask_notice got;
         {
             Notice notice(m.get_device());
+            const Released gil;
+            frp = make({rows}, at::kInt, m);
+            prp = make({rows}, at::kInt, m);
+            lrp = make({rows}, at::kInt, m);
+            nnz = make({}, at::kFloat, m);
+            ws = make({static_cast<int64_t>(ws_bytes)}, at::kByte, m);
             call("stof_mask_classify", api.mask_classify_notify, m.data_ptr(), dt, static_cast<int>(B), s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(),
                  lrp.data_ptr<int>(), nnz.data_ptr<float>(), ws.data_ptr(), ws_bytes, notice.header(), l.status, notice.record(), notice.stamp, l.stream);
             got = notice.wait(stream);
@@ -794,15 +822,18 @@ PyObject* py_sparse_storage(PyObject*, PyObject* const* a, Py_ssize_t n) {
             if (r == nullptr) throw PythonFail{};
             Py_DECREF(r);
         }
-        const at::Tensor fci = make({got.n_full}, at::kInt, m), pci = make({got.n_part}, at::kInt, m), lci = make({got.n_full + got.n_part}, at::kInt, m);
-        at::Tensor tiles = make({got.n_part > 0 ? got.n_part : 1, bm, bn}, at::kHalf, m);
-        if (got.n_part == 0) {
+        {
             const Released gil;
-            tiles.fill_(1);
+            fci = make({got.n_full}, at::kInt, m);
+            pci = make({got.n_part}, at::kInt, m);
+            lci = make({got.n_full + got.n_part}, at::kInt, m);
+            tiles = make({got.n_part > 0 ? got.n_part : 1, bm, bn}, at::kHalf, m);
+            if (got.n_part == 0) tiles.fill_(1);
+            if (got.n_full + got.n_part > 0)
+                call("stof_mask_fill", api.mask_fill, m.data_ptr(), dt, s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(),
+                     fci.data_ptr<int>(), pci.data_ptr<int>(), lci.data_ptr<int>(), got.n_part > 0 ? tiles.data_ptr() : nullptr, ws.data_ptr(), ws_bytes,
+                     l.stream);
         }
-        if (got.n_full + got.n_part > 0)
-            call("stof_mask_fill", api.mask_fill, m.data_ptr(), dt, s, ibm, ibn, frp.data_ptr<int>(), prp.data_ptr<int>(), lrp.data_ptr<int>(), fci.data_ptr<int>(),
-                 pci.data_ptr<int>(), lci.data_ptr<int>(), got.n_part > 0 ? tiles.data_ptr() : nullptr, ws.data_ptr(), ws_bytes, l.stream);
         const at::Tensor* out[8] = {&nnz, &frp, &fci, &prp, &pci, &tiles, &lrp, &lci};
         PyObject* tuple = PyTuple_New(8);
         for (int i = 0; i < 8; ++i) PyTuple_SET_ITEM(tuple, i, wrap(*out[i]));

@@ -83,9 +83,11 @@ def test_python_threads_run_while_the_library_is_in_a_call(tmp_path, monkeypatch
     idx, (q, k, v) = _index(256, 32, 40), (_rand((1, 2, 256, 64), i).cuda() for i in range(3))
     mask = torch.ones(1, 64, 64, device="cuda")
     out = torch.empty_like(q)
+    enc, hidden = _encoder(128, 2, 256, 64), _rand((1, 64, 128), 3).cuda()
+    enc(hidden)                                          # with the use below the plan is decided
     calls = {"gemm": lambda: stof_b200.gemm_bias(x, w), "gemm_ln": lambda: stof_b200.gemm_bias_residual_layernorm(x, w, None, None, None, None, 1e-5),
              "layernorm": lambda: stof_b200.bias_residual_layernorm(x), "attention": lambda: stof_b200.block_attention(q, k, v, out, *idx, 32, 32),
-             "compaction": lambda: stof_b200.get_sparse_storage(mask, 64, 64)}
+             "compaction": lambda: stof_b200.get_sparse_storage(mask, 64, 64), "stack": lambda: enc(hidden)}
     for f in calls.values():
         f()
     ticks, stop = [0], threading.Event()
@@ -217,3 +219,41 @@ def test_plan_list_gives_up_the_index_used_longest_ago(monkeypatch):
     finally:
         _lib._native = None
         _lib.native()
+
+
+def test_stacks_of_two_threads_beside_a_thread_that_computes():
+    """Two encoders on streams of their own and a Python thread that never waits: the walks, which run without the interpreter's lock,
+    give what they give alone."""
+    import threading
+    encs, xs = [_encoder(128, 2, 256, 64) for _ in range(2)], [_rand((2, 64, 128), 30 + i).cuda() for i in range(2)]
+    want = []
+    for e, x in zip(encs, xs):
+        e(x), e(x)
+        want.append(e(x).clone())
+    torch.cuda.synchronize()
+    stop, wrong = threading.Event(), []
+
+    def compute():
+        n = 0
+        while not stop.is_set():
+            n += 1
+
+    def walk(e, x, w):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(50):
+                    if not torch.equal(e(x), w):
+                        wrong.append("another result")
+        except Exception as error:
+            wrong.append(repr(error))
+
+    threads = [threading.Thread(target=walk, args=a) for a in zip(encs, xs, want)]
+    busy = threading.Thread(target=compute)
+    busy.start()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    stop.set()
+    busy.join()
+    assert not wrong, wrong[:3]
