@@ -18,6 +18,7 @@
 // What bounds it: the main loop from K = 1024 on, below that the epilogue.  With 8 epilogue warps of 128 columns each, x written back to
 // tensor memory, the residual loaded row by row (16 of every 2048 bytes per request) and releasing remote arrives, a row block of 128 took
 // 11 to 16 us whatever K was.  With residual, K = N = 768: 32768 rows 100 -> 49 us, 8192 24.1 -> 19.3; K = N = 1024: 32768 rows 133 -> 78 us.
+// (At 18 warps the cap is 96 registers; 56 bytes are spilled and 104 read back.)
 // The statistics are fp32 and taken before any rounding to fp16 (the unfused path rounds the GEMM output first).
 // Both tables and the "partials complete" barriers are double-buffered like the accumulators: a block may run at most one row block
 // ahead of its peers, because it cannot complete row block t + 1 before every peer has contributed to it; a peer's warps contribute

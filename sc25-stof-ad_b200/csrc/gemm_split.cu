@@ -18,8 +18,8 @@
 //               finishes rows r * BM / S ..: every block sends each peer that peer's rows with one bulk copy into the peer's
 //               receive buffer, which reports to the peer's barrier (reading them there with loads took 1300 - 3200 cycles, and
 //               two more cluster barriers).  No atomics, no workspace in global memory, and the order of the sum is fixed.
-// Measured (weights from HBM, back to back, against the one-block kernel): 128 rows 768 -> 768 columns 9.1 -> 3.9 us, 768 -> 3072
-// 10.5 -> 4.7 us, 3072 -> 768 22.7 -> 6.1 us.
+// Measured (weights from HBM, back to back, against the one-block kernel): 128 rows 768 -> 768 columns 8.1 -> 3.6 us, 768 -> 3072
+// 8.4 -> 4.0 us, 3072 -> 768 19.9 -> 5.9 us; more beside the dispatch in gemm_tc.cu.
 #include <atomic>
 #include "gemm_split.cuh"
 #include "stof_epilogue.cuh"

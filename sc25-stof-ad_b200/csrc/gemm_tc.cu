@@ -329,9 +329,9 @@ extern "C" int stof_gemm_bias_act(const void* a, long long lda, const void* w, l
     if (pair_mode() < 0) {
         // Few tiles: the smallest tiles that still all run at once, with K cut in two or four where it is long and that still fits
         // (gemm_split.cu; a second wave of these one-tile blocks costs more than the 128 x 256 tiles of the kernel below).
-        // Measured, weights from HBM, this kernel against the 128 x 256 one: K = 768: 128 rows x 768 columns 64 x 64 3.4 / 9.1 us,
-        // 512 x 2304 128 x 64 5.3 / 8.9, 1000 x 2304 128 x 128 7.3 / 9.0, 512 x 3072 128 x 128 7.8 / 10.5; K = 3072, 768 columns:
-        // 128 rows 64 x 64 in two parts 5.8 / 22.9, 512 rows 64 x 64 8.2 / 21.4, 1000 rows 128 x 64 10.3 / 21.1.
+        // Measured, weights from HBM, this kernel against the 128 x 256 one: K = 768: 128 rows x 768 columns 64 x 64 3.6 / 8.1 us,
+        // 512 x 2304 128 x 64 5.1 / 8.2, 1000 x 2304 128 x 128 7.1 / 8.2, 512 x 3072 128 x 128 6.8 / 8.3; K = 3072, 768 columns:
+        // 128 rows 64 x 64 in two parts 5.9 / 19.9, 512 rows 64 x 64 8.1 / 19.7, 1000 rows 128 x 64 10.6 / 19.5.
         // C over A is sound where one block reads a row of A and writes it, after its last product: with tiles as wide as the matrix.
         // (Up to 256 columns the kernel below has such tiles.)
         const bool over_a = overlap(a, ((m - 1LL) * lda + k) * 2, c, ((m - 1LL) * ldc + n) * 2);

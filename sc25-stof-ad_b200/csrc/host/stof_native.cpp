@@ -2,7 +2,7 @@
 //
 // A call of an operator costs a few microseconds of GPU time at serving sizes, so what the host does per call decides the
 // rate: the same checks and launches in Python (tensor attributes, a device context manager, ctypes with twenty arguments)
-// took 25 - 45 us per operator and 1.75 ms for the 60 launches of a 12-layer encoder on 128 tokens.  This module takes the
+// took 25 - 45 us per operator and 1.75 ms for the 72 launches of a 12-layer encoder on 128 tokens.  This module takes the
 // Python arguments once, works on at::Tensor, and calls the C ABI (include/stof_b200.h) through function pointers of the
 // library that the ctypes layer loaded; the encoder and decoder stacks walk their layers here without returning to Python.
 //

@@ -64,7 +64,8 @@ __device__ __forceinline__ void store8(__half* p, const float (&f)[8]) {
 // What bounds it: HBM and, one row at a time, the issue slots and the two reductions (590 instructions a row, 16 warps on an SM,
 // 2.7 TB/s at 32768 x 1024 from HBM).  Two rows at a time share the conversion of bias, gamma and beta (held as fp16 in registers: as
 // fp32 they alone took 64) and overlap their reductions: from HBM, 32768 rows of 768 28 -> 19 us (5.2 TB/s), of 1024 45 -> 27 us,
-// 8192 rows of 768 9.5 -> 8.0 us.  Two blocks on an SM matter more than the last registers (hidden 768: 23 us with one of 152).
+// 8192 rows of 768 9.5 -> 8.0 us.  Two blocks on an SM matter more than the last registers (hidden 768: 23 us with one of 152; at
+// hidden 1024 two rows spill 48 bytes at the cap of 128).
 template <int NCHUNK, int ROWS>
 __global__ void __launch_bounds__(LN_WARPS * 32, 2)
 layernorm_kernel(const __half* x, long long ldx, const __half* bias, const __half* residual,

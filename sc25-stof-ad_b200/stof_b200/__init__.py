@@ -2,7 +2,8 @@
 
 PyTorch supplies device memory, streams and (for multi-GPU runs) process groups; every
 computation of the two accelerated paths runs in the hand-written CUDA kernels of
-`libstof_b200.so`, reached through its C ABI with ctypes.  There is no CPU or library
+`libstof_b200.so`, reached through its C ABI: by the native host path `_stof_native.so` on every call
+of an operator, and with ctypes for plans and the rest.  There is no CPU or library
 fallback: if the shared library is missing or a tensor is not on a CUDA device that can
 be used, the call raises.
 """
