@@ -92,6 +92,11 @@ struct Released {
     Released(const Released&) = delete;
     ~Released() { if (ts != nullptr) PyEval_RestoreThread(ts); }
 };
+template <class F>
+auto released(F&& f) {
+    const Released gil;
+    return f();
+}
 template <class F, class... A>
 void call(const char* what, F* f, A... args) {
     int rc;
@@ -476,8 +481,9 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor &x = tensor_needed(a[0], "gemm"), &w = tensor_needed(a[1], "gemm");
         const at::Tensor *bias = tensor_arg(a[2], "gemm"), *res = tensor_arg(a[4], "gemm"), *out = tensor_arg(a[5], "gemm");
         for (const at::Tensor* t : {&x, &w, bias, res, out}) need_cuda(t);
+        const int epilogue = static_cast<int>(long_arg(a[3]));
         const Launch l(x);
-        const at::Tensor made = gemm_core(l, x, w, bias, static_cast<int>(long_arg(a[3])), res, out);
+        const at::Tensor made = released([&] { return gemm_core(l, x, w, bias, epilogue, res, out); });
         return out != nullptr ? same(a[5]) : wrap(made);
     });
 }
@@ -490,8 +496,9 @@ PyObject* py_gemm_ln(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor *v[4], *out = tensor_arg(a[7], "gemm_ln");
         for (int i = 0; i < 4; ++i) v[i] = tensor_arg(a[2 + i], "gemm_ln");
         for (const at::Tensor* t : {&x, &w, v[0], v[1], v[2], v[3], out}) need_cuda(t);
+        const double eps = double_arg(a[6]);
         const Launch l(x);
-        const at::Tensor made = gemm_ln_core(l, x, w, v[0], v[1], v[2], v[3], double_arg(a[6]), out);
+        const at::Tensor made = released([&] { return gemm_ln_core(l, x, w, v[0], v[1], v[2], v[3], eps, out); });
         return out != nullptr ? same(a[7]) : wrap(made);
     });
 }
@@ -504,8 +511,9 @@ PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor *v[4], *out = tensor_arg(a[6], "layernorm");
         for (int i = 0; i < 4; ++i) v[i] = tensor_arg(a[1 + i], "layernorm");
         for (const at::Tensor* t : {&x, v[0], v[1], v[2], v[3], out}) need_cuda(t);
+        const double eps = double_arg(a[5]);
         const Launch l(x);
-        const at::Tensor made = layernorm_core(l, x, v[0], v[1], v[2], v[3], double_arg(a[5]), out);
+        const at::Tensor made = released([&] { return layernorm_core(l, x, v[0], v[1], v[2], v[3], eps, out); });
         return out != nullptr ? same(a[6]) : wrap(made);
     });
 }
